@@ -304,22 +304,46 @@ void scan_exclusive(const uint32_t *in, uint32_t *out, size_t n,
     GN_CUDA(cudaStreamSynchronize(s));  // `own` is released on return
 }
 
+namespace
+{
+// u32 offsets of the sort's scratch: histograms and their scan scratch,
+// ping-pong keys, ping-pong values
+void sort_layout(size_t n, unsigned &nb, size_t &nh, size_t &tk, size_t &tv)
+{
+  nb = (unsigned)((n + kSortTile - 1) / kSortTile);
+  nh = (size_t)256 * nb;
+  tk = (nh + scan_scratch_elems(nh) + 63) / 64 * 64;  // 256-byte aligned
+  tv = tk + (n + 63) / 64 * 64;
+}
+}  // namespace
+
+size_t sort_scratch_elems(size_t n)
+{
+  unsigned nb;
+  size_t nh, tk, tv;
+  sort_layout(n, nb, nh, tk, tv);
+  return tv + n;
+}
+
 void sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in,
                 uint32_t *keys_out, uint32_t *vals_out, size_t n, int key_bits,
-                cudaStream_t s)
+                cudaStream_t s, uint32_t *scratch)
 {
   if (n == 0)
     return;
   if (n >= (1ull << 32))
     throw Error(kNotSupported, "more than 2^32 items to sort");
   const int passes = (key_bits + 7) / 8;
-  const unsigned nb = (unsigned)((n + kSortTile - 1) / kSortTile);
-  // one allocation: histograms, their scan scratch, ping-pong keys / values
-  const size_t nh = (size_t)256 * nb, nsc = scan_scratch_elems(nh);
-  const size_t off_tk = (nh + nsc + 63) / 64 * 64;  // 256-byte aligned
-  const size_t off_tv = off_tk + (n + 63) / 64 * 64;
-  DeviceBuffer work((off_tv + n) * sizeof(uint32_t));
-  uint32_t *hist = work.as<uint32_t>(), *scratch = hist + nh;
+  unsigned nb;
+  size_t nh, off_tk, off_tv;
+  sort_layout(n, nb, nh, off_tk, off_tv);
+  DeviceBuffer own;
+  if (!scratch)
+  {
+    own.reset(sort_scratch_elems(n) * sizeof(uint32_t));
+    scratch = own.as<uint32_t>();
+  }
+  uint32_t *hist = scratch, *sums = hist + nh;
   uint32_t *tk = hist + off_tk, *tv = hist + off_tv;
   // ping-pong so that the last pass lands in *_out
   const uint32_t *ki = keys_in, *vi = vals_in;
@@ -330,18 +354,19 @@ void sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in,
     uint32_t *vo = to_out ? vals_out : tv;
     k_radix_hist<<<nb, kSortThreads, 0, s>>>(ki, n, 8 * p, hist);
     GN_LAUNCH_CHECK("radix hist");
-    scan_exclusive(hist, hist, nh, s, scratch);
+    scan_exclusive(hist, hist, nh, s, sums);
     k_radix_scatter<<<nb, kSortThreads, 0, s>>>(ki, vi, ko, vo, n, 8 * p,
                                                 hist);
     GN_LAUNCH_CHECK("radix scatter");
     ki = ko;
     vi = vo;
   }
-  GN_CUDA(cudaStreamSynchronize(s));  // `work` is released on return
+  if (own.get())
+    GN_CUDA(cudaStreamSynchronize(s));  // `own` is released on return
 }
 
 void histogram_offsets(const uint32_t *keys, size_t n, uint32_t bins,
-                       uint32_t *offsets, cudaStream_t s)
+                       uint32_t *offsets, cudaStream_t s, uint32_t *scratch)
 {
   GN_CUDA(cudaMemsetAsync(offsets, 0, (size_t)(bins + 1) * sizeof(uint32_t),
                           s));
@@ -350,7 +375,7 @@ void histogram_offsets(const uint32_t *keys, size_t n, uint32_t bins,
     k_count_keys<<<grid_for(n, 256, 4096), 256, 0, s>>>(keys, n, offsets);
     GN_LAUNCH_CHECK("count keys");
   }
-  scan_exclusive(offsets, offsets, (size_t)bins + 1, s);
+  scan_exclusive(offsets, offsets, (size_t)bins + 1, s, scratch);
 }
 
 void assign_sectors(const float *traj, uint32_t M, const Geo &g,
@@ -377,7 +402,7 @@ size_t build_interp_matrix(const float *traj_sorted,
                            const uint32_t *sector_sorted, uint32_t M,
                            const Geo &g, const float *lut,
                            DeviceBuffer &row_off, DeviceBuffer &nz,
-                           cudaStream_t s)
+                           BuildWork &work, cudaStream_t s)
 {
   const uint32_t G = (uint32_t)g.grid_count;
   row_off.reset((size_t)(G + 1) * sizeof(uint32_t));
@@ -388,37 +413,39 @@ size_t build_interp_matrix(const float *traj_sorted,
     return 0;
   }
   const size_t nsc = scan_scratch_elems((size_t)M + 1);
-  DeviceBuffer count(((size_t)M + 1 + nsc) * sizeof(uint32_t));
-  GN_CUDA(cudaMemsetAsync(count.get(), 0, (size_t)(M + 1) * 4, s));
+  work.counts.ensure(((size_t)M + 1 + nsc) * sizeof(uint32_t));
+  uint32_t *count = work.counts.as<uint32_t>();
+  GN_CUDA(cudaMemsetAsync(count, 0, (size_t)(M + 1) * 4, s));
   const unsigned nb = grid_for(M, 256, 8192);
   k_interp_pairs<false><<<nb, 256, 0, s>>>(traj_sorted, sector_sorted, M, g,
-                                           lut, count.as<uint32_t>(), nullptr,
-                                           nullptr, nullptr, nullptr);
+                                           lut, count, nullptr, nullptr,
+                                           nullptr, nullptr);
   GN_LAUNCH_CHECK("interp count");
-  scan_exclusive(count.as<uint32_t>(), count.as<uint32_t>(), (size_t)M + 1,
-                 s, count.as<uint32_t>() + M + 1);
+  scan_exclusive(count, count, (size_t)M + 1, s, count + M + 1);
   uint32_t total = 0;
-  GN_CUDA(cudaMemcpyAsync(&total, count.as<uint32_t>() + M, sizeof(uint32_t),
+  GN_CUDA(cudaMemcpyAsync(&total, count + M, sizeof(uint32_t),
                           cudaMemcpyDeviceToHost, s));
   GN_CUDA(cudaStreamSynchronize(s));
   const size_t n = total;
-  DeviceBuffer keys(n * 4 + 4), ids(n * 4 + 4), pairs(n * 8 + 8);
-  k_interp_pairs<true><<<nb, 256, 0, s>>>(
-      traj_sorted, sector_sorted, M, g, lut, nullptr, count.as<uint32_t>(),
-      keys.as<uint32_t>(), ids.as<uint32_t>(), pairs.as<uint2>());
+  // pairs | keys | ids | sorted keys | sorted ids | sort (then scan) scratch
+  const size_t np = (n + 63) / 64 * 64;
+  work.tables.ensure((6 * np + std::max(sort_scratch_elems(n),
+                                        scan_scratch_elems((size_t)G + 1))) *
+                         sizeof(uint32_t) +
+                     16);
+  uint2 *pairs = work.tables.as<uint2>();
+  uint32_t *keys = reinterpret_cast<uint32_t *>(pairs + np), *ids = keys + np;
+  uint32_t *skeys = ids + np, *sids = skeys + np, *scratch = sids + np;
+  k_interp_pairs<true><<<nb, 256, 0, s>>>(traj_sorted, sector_sorted, M, g,
+                                          lut, nullptr, count, keys, ids,
+                                          pairs);
   GN_LAUNCH_CHECK("interp fill");
-  count.release();
-  DeviceBuffer skeys(n * 4 + 4), sids(n * 4 + 4);
-  sort_pairs(keys.as<uint32_t>(), ids.as<uint32_t>(), skeys.as<uint32_t>(),
-             sids.as<uint32_t>(), n, bits_for(G ? G - 1 : 0), s);
-  keys.release();
-  ids.release();
+  sort_pairs(keys, ids, skeys, sids, n, bits_for(G ? G - 1 : 0), s, scratch);
   nz.reset(n * 8 + 8);
-  k_gather_pairs<<<grid_for(n, 256, 8192), 256, 0, s>>>(
-      sids.as<uint32_t>(), pairs.as<uint2>(), n, nz.as<uint2>());
+  k_gather_pairs<<<grid_for(n, 256, 8192), 256, 0, s>>>(sids, pairs, n,
+                                                        nz.as<uint2>());
   GN_LAUNCH_CHECK("interp gather");
-  histogram_offsets(skeys.as<uint32_t>(), n, G, row_off.as<uint32_t>(), s);
-  GN_CUDA(cudaStreamSynchronize(s));
+  histogram_offsets(skeys, n, G, row_off.as<uint32_t>(), s, scratch);
   return n;
 }
 

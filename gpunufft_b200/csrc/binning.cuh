@@ -20,14 +20,26 @@ void scan_exclusive(const uint32_t *in, uint32_t *out, size_t n,
 size_t scan_scratch_elems(size_t n);
 
 // Stable LSD radix sort of (key, value) pairs on the low `key_bits` bits of
-// the keys.  Sorted output ends in keys_out / vals_out.
+// the keys.  Sorted output ends in keys_out / vals_out.  `scratch` (device,
+// sort_scratch_elems(n) u32, or NULL): as for scan_exclusive.
 void sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in,
                 uint32_t *keys_out, uint32_t *vals_out, size_t n, int key_bits,
-                cudaStream_t s);
+                cudaStream_t s, uint32_t *scratch = nullptr);
+size_t sort_scratch_elems(size_t n);
 
-// Counts of `n` keys in [0, bins) -> offsets[bins + 1] (exclusive scan).
+// Counts of `n` keys in [0, bins) -> offsets[bins + 1] (exclusive scan;
+// scratch of scan_scratch_elems(bins + 1) as for scan_exclusive).
 void histogram_offsets(const uint32_t *keys, size_t n, uint32_t bins,
-                       uint32_t *offsets, cudaStream_t s);
+                       uint32_t *offsets, cudaStream_t s,
+                       uint32_t *scratch = nullptr);
+
+// Device memory of the table builders: one pair of buffers serves a plan's
+// builders in turn (an allocation or a release each costs a device
+// synchronisation).
+struct BuildWork
+{
+  DeviceBuffer counts, tables;
+};
 
 // Sector of every sample, original order (assignSectors,
 // gpuNUFFT_operator_factory.cpp:128-181; precomp_kernels.cu:8-45).
@@ -51,7 +63,7 @@ size_t build_interp_matrix(const float *traj_sorted,
                            const uint32_t *sector_sorted, uint32_t M,
                            const Geo &g, const float *lut,
                            DeviceBuffer &row_off, DeviceBuffer &nz,
-                           cudaStream_t s);
+                           BuildWork &work, cudaStream_t s);
 
 // Per (y, x) column of the grid, the range [lo, hi] of z cells that carry
 // interpolation weights (widened by one; lo > hi when none): the forward

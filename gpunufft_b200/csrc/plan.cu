@@ -34,6 +34,7 @@
 #include "gridding.cuh"
 #include "hostcopy.hpp"
 #include "planview.hpp"
+#include "tilespread.cuh"
 #include "tma.cuh"
 #include "trajgrad.cuh"
 
@@ -95,6 +96,7 @@ struct gnufft_plan
   DeviceBuffer roots[3];      // DFT roots per axis (pruned transforms)
   DeviceBuffer zrange;        // per (y, x) column: z rows with weights
   DeviceBuffer ztiles;        // column tiles holding a z range
+  TileTables tiles;           // records of the tile spread (adjoint)
   int n_ztiles = 0;
   float dlut_mult = 0.f;
   size_t nnz = 0;
@@ -104,6 +106,7 @@ struct gnufft_plan
 
   // per-call scratch (grow-only)
   DeviceBuffer ks, grid, stage_in, stage_out, one_sens, fft_a, fft_b;
+  DeviceBuffer tile_part;  // partial tiles of the tile spread
   std::map<int, cufftHandle> fft;
 
   // timing
@@ -148,8 +151,8 @@ struct gnufft_plan
                                   &stage_out,   &one_sens,    &fft_a,
                                   &fft_b,       &dlut,        &roots[0],
                                   &roots[1],    &roots[2],    &zrange,
-                                  &ztiles};
-    size_t s = 0;
+                                  &ztiles,      &tile_part};
+    size_t s = tiles.bytes();
     for (auto *b : bufs)
       s += b->bytes();
     return s;
@@ -380,9 +383,11 @@ void set_sens_host(gnufft_plan &p, const void *sens, uint32_t n_coils)
 void finish_tables(gnufft_plan &p)
 {
   // interpolation matrix (adjoint) and forward work items
+  BuildWork work;
   p.nnz = build_interp_matrix(p.traj_sorted.as<float>(),
                               p.sec_sorted.as<uint32_t>(), p.M, p.g,
-                              p.lut.as<float>(), p.w_rows, p.w_nz, p.stream);
+                              p.lut.as<float>(), p.w_rows, p.w_nz, work,
+                              p.stream);
   build_items(p);
   if (p.dim == 3 && forward_pairs(p.g, 0))
   {
@@ -395,6 +400,9 @@ void finish_tables(gnufft_plan &p)
   p.di_inv.reset((size_t)p.M * sizeof(uint32_t) + 4);
   launch_invert_permutation(p.di.as<uint32_t>(), p.M, p.di_inv.as<uint32_t>(),
                             p.stream);
+  if (p.pruned && tile_spread_supported(p.g))
+    build_tile_tables(p.traj_sorted.as<float>(), p.sec_sorted.as<uint32_t>(),
+                      p.M, p.g, p.lut.as<float>(), p.tiles, work, p.stream);
   if (p.pruned && p.dim == 3)
     build_column_ranges(p.w_rows.as<uint32_t>(), p.g, p.zrange, p.ztiles,
                         p.n_ztiles, p.stream);
@@ -601,6 +609,41 @@ std::array<const float2 *, 3> root_ptrs(const gnufft_plan &p)
           p.roots[2].as<float2>()};
 }
 
+// The adjoint of C coils spreads by register columns (tilespread.cuh)
+// instead of the CSR product.  It costs two to four launches more and issues
+// the same instructions per record for 8 coils as for 32; the CSR kernels
+// give a coil count's lanes several entries at once but pay per (sample,
+// cell) pair.  Whole adjoints, CSR -> columns, us on a B200 (M samples,
+// entries x lanes = CSR entries times coil lanes):
+//   3-D, 27 entries a sample: 32^3 image, 16 / 32 coils (14 / 28 M entries x
+//   lanes) 64 -> 65, 121 -> 102; 64^3, 3 / 8 / 32 coils (28 / 57 / 226 M)
+//   174 -> 133, 237 -> 186, 603 -> 491; 128^3, 32 coils 3899 -> 2928; kernel
+//   width 7 at 64^3 653 -> 339 (4 coils)
+//   2-D, 9 entries: 128^2, 8 / 16 / 32 coils (4 / 7 / 15 M) 33 -> 36,
+//   45 -> 41, 70 -> 52; 256^2, 4 / 8 / 16 / 32 coils (7 / 15 / 30 / 59 M)
+//   46 -> 51, 62 -> 70, 126 -> 104, 211 -> 156; 512^2 (rows of 1024, one CSR
+//   block per SM), 3 / 32 coils 199 -> 159, 1207 -> 605; kernel widths 4 / 5
+//   at 256^2, 3 coils (3 / 4 M) 44 -> 41, 51 -> 43.
+bool tile_path(const gnufft_plan &p, uint32_t C)
+{
+  if (!p.pruned || !p.copy_err_d || !p.tiles.ready() || C <= 2 ||
+      !tile_xpass_supported(p.g))
+    return false;
+  const double work = (double)p.nnz * spmm_coil_group((int)C) *
+                      ((C + 31) / 32);
+  if (p.dim == 3)
+    return work >= 20e6;
+  if (p.g.G[0] > 512 || p.g.kw > 3)
+    return work >= 3e6;
+  return C > 8 && work >= 6e6;
+}
+
+// Complex elements of the adjoint's x-transformed rows.
+size_t xrows_elems(const Geo &g, uint32_t C)
+{
+  return (size_t)C * g.G[2] * g.G[1] * g.N[0];
+}
+
 // All coils of the call in one pass.
 void adjoint_batched(gnufft_plan &p, const float2 *k, float2 *img, uint32_t C,
                      int stage, cudaStream_t s, const float2 *sens,
@@ -614,10 +657,12 @@ void adjoint_batched(gnufft_plan &p, const float2 *k, float2 *img, uint32_t C,
   p.ks.ensure((size_t)p.M * CP * sizeof(float2));
   const bool conv = stage == GNUFFT_CONVOLUTION ||
                     stage == GNUFFT_DENSITY_ESTIMATION;
+  const bool tiled = !conv && tile_path(p, C);
   float2 *grid = img;
   if (!conv)
   {
-    p.grid.ensure((size_t)C * g.grid_count * sizeof(float2));
+    p.grid.ensure((size_t)(tiled ? tile_grid_pitch((int)C) : (int)C) *
+                  g.grid_count * sizeof(float2));
     grid = p.grid.as<float2>();
   }
   p.mark(0, s);
@@ -627,6 +672,33 @@ void adjoint_batched(gnufft_plan &p, const float2 *k, float2 *img, uint32_t C,
   p.launches += 1;
   p.mark(1, s);
   p.mark(2, s);
+  if (tiled)
+  {  // spread by register tiles into a coil-interleaved grid, inverse x
+     // transform to coil-major rows, then y and z
+    check_copy_err(p);
+    ensure_pruned(p, C, s);
+    p.fft_b.ensure(xrows_elems(g, C) * sizeof(float2));
+    p.tile_part.ensure(tile_partial_elems(p.tiles, g, (int)C) * sizeof(float2));
+    p.launches += launch_tile_spread(p.tiles, p.ks.as<float2>(), CP, g,
+                                     (int)C, grid, p.tile_part.as<float2>(),
+                                     s);
+    p.mark(3, s);
+    p.mark(4, s);
+    launch_tile_xpass(p.tiles, grid, g, (int)C, p.roots[0].as<float2>(),
+                      p.fft_b.as<float2>(), copy_wait(p), s);
+    // the spread's grid is free once its rows are transformed: it takes the
+    // y pass's output
+    launch_pruned_adjoint_xfirst(
+        p.fft_b.as<float2>(), p.deapo.as<float>(),
+        stage == GNUFFT_DEAPODIZATION ? sens : nullptr, g, (int)C,
+        stage == GNUFFT_FFT ? 1 : 2, accumulate, root_ptrs(p).data(), grid,
+        p.fft_a.as<float2>(), img, s, copy_wait(p));
+    p.launches += g.dim;
+    p.mark(5, s);
+    p.mark(6, s);
+    p.mark(7, s);
+    return;
+  }
   if (p.pruned && !conv)
   {  // spread whole grid rows with the inverse x transform fused (the grid
      // buffer receives only the cropped x outputs), then y and z
@@ -821,11 +893,16 @@ size_t call_scratch_bytes(const gnufft_plan &p, uint32_t C)
   const size_t G = (size_t)g.grid_count, f2 = sizeof(float2);
   const size_t cg = (size_t)spmm_coil_group((int)C);
   const size_t CP = (C + cg - 1) / cg * cg;
-  size_t b = (size_t)p.M * CP * f2 + (size_t)(C + 1) / 2 * 2 * G * f2;
+  const bool tiled = tile_path(p, C);
+  const size_t pitch = std::max<size_t>(
+      (C + 1) / 2 * 2, tiled ? (size_t)tile_grid_pitch((int)C) : 0);
+  size_t b = (size_t)p.M * CP * f2 + pitch * G * f2;
   if (p.pruned)
     b += (pruned_scratch_a(g, (int)C) +
-          std::max(pruned_scratch_b(g, (int)C),
-                   pruned_scratch_xfirst(g, (int)C))) *
+          std::max({pruned_scratch_b(g, (int)C),
+                    pruned_scratch_xfirst(g, (int)C),
+                    tiled ? xrows_elems(g, C) : (size_t)0}) +
+          (tiled ? tile_partial_elems(p.tiles, g, (int)C) : 0)) *
          f2;
   else
     b += (size_t)C * G * f2;
@@ -834,7 +911,8 @@ size_t call_scratch_bytes(const gnufft_plan &p, uint32_t C)
 
 size_t held_scratch_bytes(const gnufft_plan &p)
 {
-  return p.ks.bytes() + p.grid.bytes() + p.fft_a.bytes() + p.fft_b.bytes();
+  return p.ks.bytes() + p.grid.bytes() + p.fft_a.bytes() + p.fft_b.bytes() +
+         p.tile_part.bytes();
 }
 
 // Coils per pass so that a pass's scratch fits the plan's memory limit, or

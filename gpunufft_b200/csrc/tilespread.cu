@@ -1,0 +1,1192 @@
+// Adjoint spread by register columns (see tilespread.cuh).
+//
+// What bounds it: instruction issue.  Per (sample, column) record a warp
+// reads one k-space row (8 bytes per coil) and 64 bytes of weights and
+// issues about 70 instructions, 24 of them paired multiply-adds; a column is
+// written once.  3-D 128^3, 32 coils, 2.1 M samples on a B200: 0.92 ms for
+// the spread (3.4 records a sample) + 0.07 ms for the columns of several
+// chunks + 0.93 ms for the x transform (4.4 GB), against 2.87 ms for the CSR
+// product with the x transform fused, whose 27 gathers a sample wait on one
+// another.  Tiles of 4 x 4 x 4 cells, every row of a tile predicated per
+// record, took 1.54 ms (118 instructions a record, 12 warps an SM); 4 x 4 x
+// 2 cells 1.46 ms (4.5 records a sample); walking the planes needs no test
+// per row and keeps only the planes of one footprint in registers.
+#include "tilespread.cuh"
+
+#include <algorithm>
+#include <type_traits>
+#include <vector>
+
+#include "binning.cuh"
+#include "f32x2.cuh"
+#include "fftcore.cuh"
+#include "footprint.cuh"
+
+namespace gnufft
+{
+namespace
+{
+// ------------------------------------------------------------------------
+// column numbering
+// ------------------------------------------------------------------------
+// A column is X x R cells across and SEG cells along the walked axis
+// (3-D z, 2-D y).  Columns of one super column (3-D 2 x 4, 2-D 2 x 1) are
+// consecutive, so that the warps of a block and blocks launched together
+// read the same k-space rows.
+template <int DIM> struct Tile
+{
+  static constexpr int X = DIM == 3 ? 4 : 8, R = DIM == 3 ? 2 : 1;
+  static constexpr int SEG = DIM == 3 ? 16 : 8;  // planes per column
+  static constexpr int Y = DIM == 3 ? R : SEG, Z = DIM == 3 ? SEG : 1;
+  static constexpr int CELLS = X * Y * Z;
+  static constexpr int SX = 2, SY = DIM == 3 ? 4 : 1;
+  static constexpr int PER = SX * SY;
+};
+
+// The record of a (sample, column) pair, in 4-byte words: x weights [X] |
+// products of the walked axis's and (3-D) the y weights [R][PW] | sample |
+// first plane + (planes << 8) | padding to 16 bytes.  PW: planes that a
+// footprint can meet.
+template <int DIM, int PW> struct Rec
+{
+  static constexpr int W0 = Tile<DIM>::X, TW = W0 + Tile<DIM>::R * PW;
+  static constexpr int WORDS = (TW + 2 + 3) / 4 * 4;
+};
+
+struct TileDims
+{
+  int nx, ny, nz;     // columns per axis
+  int sx, sy;         // super columns
+};
+
+template <int DIM> __host__ __device__ TileDims tile_dims(const Geo &g)
+{
+  using T = Tile<DIM>;
+  TileDims d;
+  d.nx = (g.G[0] + T::X - 1) / T::X;
+  d.ny = (g.G[1] + T::Y - 1) / T::Y;
+  d.nz = (g.G[2] + T::Z - 1) / T::Z;
+  d.sx = (d.nx + T::SX - 1) / T::SX;
+  d.sy = (d.ny + T::SY - 1) / T::SY;
+  return d;
+}
+
+template <int DIM>
+__host__ __device__ uint32_t tile_id(const TileDims &d, int x, int y, int z)
+{
+  using T = Tile<DIM>;
+  const uint32_t s = ((uint32_t)z * d.sy + y / T::SY) * d.sx + x / T::SX;
+  return s * T::PER + (y % T::SY) * T::SX + x % T::SX;
+}
+
+template <int DIM>
+__host__ __device__ void tile_of_id(const TileDims &d, uint32_t id, int &x,
+                                    int &y, int &z)
+{
+  using T = Tile<DIM>;
+  uint32_t s = id / T::PER, r = id % T::PER;
+  x = (int)(s % d.sx) * T::SX + (int)(r % T::SX);
+  s /= d.sx;
+  y = (int)(s % d.sy) * T::SY + (int)(r / T::SX);
+  z = (int)(s / d.sy);
+}
+
+// ------------------------------------------------------------------------
+// plan-time tables
+// ------------------------------------------------------------------------
+// Tiles that one axis's footprint cells meet, in cell order (the cells are
+// cyclically consecutive and fewer than the axis is long, so each tile is
+// met in one run), and the first cell in each.
+__device__ __forceinline__ int axis_tiles(const int *cell, int n, int edge,
+                                          int *tile, int *first)
+{
+  int m = 0;
+  for (int e = 0; e < n; ++e)
+  {
+    const int t = cell[e] / edge;
+    if (m == 0 || tile[m - 1] != t)
+    {
+      first[m] = cell[e] - t * edge;
+      tile[m++] = t;
+    }
+  }
+  return m;
+}
+
+__device__ __forceinline__ void sample_axes(const float *traj_sorted,
+                                            uint32_t sector, uint32_t M,
+                                            uint32_t t, const Geo &g,
+                                            const float *lut,
+                                            int (*cell)[kSlots],
+                                            float (*w)[kSlots], int *n)
+{
+  int sa[3];
+  sa[0] = (int)(sector % (uint32_t)g.S[0]);
+  const uint32_t r = sector / (uint32_t)g.S[0];
+  sa[1] = (int)(r % (uint32_t)g.S[1]);
+  sa[2] = (int)(r / (uint32_t)g.S[1]);
+  n[2] = 1;
+  cell[2][0] = 0;
+  w[2][0] = 1.0f;
+  for (int a = 0; a < g.dim; ++a)
+    n[a] = axis_footprint(traj_sorted[(size_t)a * M + t], a, sa[a], g, lut,
+                          cell[a], w[a]);
+}
+
+// FILL false: count[t] = columns the footprint of sorted sample t meets.
+// FILL true: one (column * SEG + first plane, sample) pair per column
+// from position count[t] on.
+template <int DIM, bool FILL>
+__global__ void k_tile_pairs(const float *__restrict__ traj_sorted,
+                             const uint32_t *__restrict__ sector, uint32_t M,
+                             Geo g, const float *__restrict__ lut,
+                             uint32_t *__restrict__ count,
+                             uint32_t *__restrict__ keys,
+                             uint32_t *__restrict__ vals)
+{
+  using T = Tile<DIM>;
+  const TileDims d = tile_dims<DIM>(g);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < M;
+       t += gridDim.x * blockDim.x)
+  {
+    int cell[3][kSlots], n[3], tl[3][kSlots], f[3][kSlots], m[3];
+    float w[3][kSlots];
+    sample_axes(traj_sorted, sector[t], M, t, g, lut, cell, w, n);
+    m[0] = axis_tiles(cell[0], n[0], T::X, tl[0], f[0]);
+    m[1] = axis_tiles(cell[1], n[1], T::Y, tl[1], f[1]);
+    m[2] = DIM == 3 ? axis_tiles(cell[2], n[2], T::Z, tl[2], f[2]) : 1;
+    if (DIM == 2)
+      tl[2][0] = 0;
+    if (!FILL)
+    {
+      count[t] = (uint32_t)(m[0] * m[1] * m[2]);
+      continue;
+    }
+    uint32_t p = count[t];
+    for (int z = 0; z < m[2]; ++z)
+      for (int y = 0; y < m[1]; ++y)
+        for (int x = 0; x < m[0]; ++x)
+        {
+          keys[p] = tile_id<DIM>(d, tl[0][x], tl[1][y], tl[2][z]) * T::SEG +
+                    (uint32_t)(DIM == 3 ? f[2][z] : f[1][y]);
+          vals[p] = t;
+          ++p;
+        }
+  }
+}
+
+template <int DIM, int PW>
+__global__ void k_tile_records(const float *__restrict__ traj_sorted,
+                               const uint32_t *__restrict__ sector,
+                               uint32_t M, Geo g,
+                               const float *__restrict__ lut,
+                               const uint32_t *__restrict__ key,
+                               const uint32_t *__restrict__ sample,
+                               uint32_t n_rec, float *__restrict__ recs)
+{
+  using T = Tile<DIM>;
+  using R = Rec<DIM, PW>;
+  const TileDims d = tile_dims<DIM>(g);
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n_rec;
+       e += gridDim.x * blockDim.x)
+  {
+    const uint32_t t = sample[e];
+    const int z0 = (int)(key[e] % T::SEG);
+    int cell[3][kSlots], n[3], at[3];
+    float w[3][kSlots];
+    sample_axes(traj_sorted, sector[t], M, t, g, lut, cell, w, n);
+    tile_of_id<DIM>(d, key[e] / T::SEG, at[0], at[1], at[2]);
+    float *r = recs + (size_t)e * R::WORDS;
+    for (int i = 0; i < R::WORDS; ++i)
+      r[i] = 0.f;
+    for (int k = 0; k < n[0]; ++k)
+      if (cell[0][k] / T::X == at[0])
+        r[cell[0][k] % T::X] = w[0][k];
+    constexpr int A = DIM - 1;  // the walked axis
+
+    int planes = 0;
+    for (int k = 0; k < n[A]; ++k)
+    {
+      if (cell[A][k] / T::SEG != at[A])
+        continue;
+      const int p = cell[A][k] % T::SEG - z0;
+      planes = p + 1;
+      if (DIM == 2)
+        r[R::W0 + p] = w[1][k];
+      else
+        for (int q = 0; q < n[1]; ++q)
+          if (cell[1][q] / T::R == at[1])
+            r[R::W0 + (cell[1][q] % T::R) * PW + p] =
+                __fmul_rn(w[2][k], w[1][q]);
+    }
+    r[R::TW] = __uint_as_float(t);
+    r[R::TW + 1] = __uint_as_float((uint32_t)z0 | ((uint32_t)planes << 8));
+  }
+}
+
+// Columns of up to this many chunks are reduced by one thread per element.
+constexpr uint32_t kFewSlots = 8;
+
+// Per column (offsets off[column * SEG + first plane] of its records):
+// its chunks (runs of at most K records), whether it has several, and its
+// occupancy bit.
+template <int DIM, bool FILL>
+__global__ void k_tile_chunks(const uint32_t *__restrict__ off,
+                              const uint32_t *__restrict__ key,
+                              uint32_t n_ids, uint32_t K, int PW, Geo g,
+                              uint32_t *__restrict__ n_ch,
+                              uint32_t *__restrict__ n_mu,
+                              uint32_t *__restrict__ n_my,
+                              uint32_t *__restrict__ n_sl,
+                              TileChunk *__restrict__ chunks,
+                              uint4 *__restrict__ multi,
+                              uint32_t *__restrict__ occ, int occ_words)
+{
+  using T = Tile<DIM>;
+  const TileDims d = tile_dims<DIM>(g);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_ids;
+       i += gridDim.x * blockDim.x)
+  {
+    const uint32_t b = off[(size_t)i * T::SEG],
+                   e = off[(size_t)(i + 1) * T::SEG];
+    const uint32_t c = (e - b + K - 1) / K;
+    if (!FILL)
+    {
+      n_ch[i] = c;
+      n_mu[i] = c > 1 && c <= kFewSlots ? 1u : 0u;
+      n_my[i] = c > kFewSlots ? 1u : 0u;
+      n_sl[i] = c > 1 ? c : 0u;
+      continue;
+    }
+    if (c == 0)
+      continue;
+    for (uint32_t q = 0; q < c; ++q)
+    {  // equal shares
+      TileChunk ch;
+      ch.tile = i;
+      ch.begin = b + (uint32_t)((unsigned long long)(e - b) * q / c);
+      ch.end = b + (uint32_t)((unsigned long long)(e - b) * (q + 1) / c);
+      ch.slot = c > 1 ? (int)(n_sl[i] + q) : -1;
+      ch.p0 = 0;
+      ch.p1 = T::SEG;
+      if (c > 1)
+      {  // the planes its records meet
+        ch.p0 = key[ch.begin] % T::SEG;
+        ch.p1 = min((uint32_t)T::SEG, key[ch.end - 1] % T::SEG + PW);
+      }
+      ch.pad[0] = ch.pad[1] = 0;
+      chunks[n_ch[i] + q] = ch;
+    }
+    if (c > 1)  // columns of few slots first, then those of many
+      multi[c > kFewSlots ? n_mu[n_ids] + n_my[i] : n_mu[i]] =
+          make_uint4(i, n_sl[i], c, n_ch[i]);
+    int x, y, z;
+    tile_of_id<DIM>(d, i, x, y, z);
+    atomicOr(&occ[((size_t)z * d.ny + y) * occ_words + (x >> 5)],
+             1u << (x & 31));
+  }
+}
+
+int tile_x(const Geo &g) { return g.dim == 3 ? Tile<3>::X : Tile<2>::X; }
+
+int occ_words_of(const Geo &g)
+{
+  const int tx = tile_x(g);
+  return ((g.G[0] + tx - 1) / tx + 31) / 32;
+}
+
+template <int DIM, int PW>
+void build_tables(const float *traj_sorted, const uint32_t *sector,
+                  uint32_t M, const Geo &g, const float *lut, TileTables &t,
+                  BuildWork &work, cudaStream_t s)
+{
+  using T = Tile<DIM>;
+  const TileDims d = tile_dims<DIM>(g);
+  const uint32_t n_ids = (uint32_t)d.sx * d.sy * d.nz * T::PER;
+  const uint32_t n_keys = n_ids * T::SEG;
+  const int ow = occ_words_of(g);
+  const size_t occ_bytes = (size_t)d.ny * d.nz * ow * 4;
+  t.occ.reset(occ_bytes);
+  GN_CUDA(cudaMemsetAsync(t.occ.get(), 0, occ_bytes, s));
+  work.counts.ensure(
+      ((size_t)M + 1 + scan_scratch_elems((size_t)M + 1)) * 4);
+  uint32_t *cnt = work.counts.as<uint32_t>();
+  GN_CUDA(cudaMemsetAsync(cnt, 0, ((size_t)M + 1) * 4, s));
+  const unsigned nb = grid_for(M, 256, 8192);
+  k_tile_pairs<DIM, false><<<nb, 256, 0, s>>>(traj_sorted, sector, M, g, lut,
+                                              cnt, nullptr, nullptr);
+  GN_LAUNCH_CHECK("column pair count");
+  scan_exclusive(cnt, cnt, (size_t)M + 1, s, cnt + M + 1);
+  uint32_t n = 0;
+  GN_CUDA(cudaMemcpyAsync(&n, cnt + M, 4, cudaMemcpyDeviceToHost, s));
+  GN_CUDA(cudaStreamSynchronize(s));
+  if (n == 0)
+    return;
+  // pairs, sorted pairs, per-column counts, sort (then scan) scratch
+  const size_t np = ((size_t)n + 63) / 64 * 64;
+  const size_t nk = ((size_t)n_keys + 1 + 63) / 64 * 64;
+  const size_t ni = ((size_t)n_ids + 1 + 63) / 64 * 64;
+  work.tables.ensure((4 * np + nk + 4 * ni +
+                      std::max(sort_scratch_elems(n),
+                               scan_scratch_elems((size_t)n_keys + 1))) *
+                     4);
+  uint32_t *keys = work.tables.as<uint32_t>(), *vals = keys + np;
+  uint32_t *skeys = vals + np, *svals = skeys + np;
+  uint32_t *off = svals + np, *ch = off + nk, *mu = ch + ni, *my = mu + ni,
+           *sl = my + ni, *scratch = sl + ni;
+  k_tile_pairs<DIM, true><<<nb, 256, 0, s>>>(traj_sorted, sector, M, g, lut,
+                                             cnt, keys, vals);
+  GN_LAUNCH_CHECK("column pairs");
+  int bits = 1;
+  while (bits < 32 && ((n_keys - 1) >> bits))
+    ++bits;
+  sort_pairs(keys, vals, skeys, svals, n, bits, s, scratch);
+  t.recs.reset((size_t)n * Rec<DIM, PW>::WORDS * 4);
+  k_tile_records<DIM, PW><<<grid_for(n, 256, 148 * 64), 256, 0, s>>>(
+      traj_sorted, sector, M, g, lut, skeys, svals, n, t.recs.as<float>());
+  GN_LAUNCH_CHECK("column records");
+  // chunk length: a few times as many chunks as there are resident warps,
+  // within bounds that keep the per-chunk column write cheap
+  const uint32_t K = std::min<uint32_t>(512, std::max<uint32_t>(128, n / 8192));
+  GN_CUDA(cudaMemsetAsync(ch, 0, 4 * ni * 4, s));
+  histogram_offsets(skeys, n, n_keys, off, s, scratch);
+  const unsigned nt = grid_for(n_ids, 256, 8192);
+  k_tile_chunks<DIM, false><<<nt, 256, 0, s>>>(off, skeys, n_ids, K, PW, g,
+                                               ch, mu, my, sl, nullptr,
+                                               nullptr, nullptr, ow);
+  GN_LAUNCH_CHECK("column chunk count");
+  scan_exclusive(ch, ch, (size_t)n_ids + 1, s, scratch);
+  scan_exclusive(mu, mu, (size_t)n_ids + 1, s, scratch);
+  scan_exclusive(my, my, (size_t)n_ids + 1, s, scratch);
+  scan_exclusive(sl, sl, (size_t)n_ids + 1, s, scratch);
+  uint32_t tot[4];
+  GN_CUDA(cudaMemcpyAsync(&tot[0], ch + n_ids, 4, cudaMemcpyDeviceToHost, s));
+  GN_CUDA(cudaMemcpyAsync(&tot[1], mu + n_ids, 4, cudaMemcpyDeviceToHost, s));
+  GN_CUDA(cudaMemcpyAsync(&tot[2], sl + n_ids, 4, cudaMemcpyDeviceToHost, s));
+  GN_CUDA(cudaMemcpyAsync(&tot[3], my + n_ids, 4, cudaMemcpyDeviceToHost, s));
+  GN_CUDA(cudaStreamSynchronize(s));
+  t.n_chunks = (int)tot[0];
+  t.n_few = (int)tot[1];
+  t.n_many = (int)tot[3];
+  t.n_slots = (int)tot[2];
+  t.chunks.reset((size_t)tot[0] * sizeof(TileChunk));
+  t.multi.reset(std::max<size_t>(tot[1] + tot[3], 1) * sizeof(uint4));
+  k_tile_chunks<DIM, true><<<nt, 256, 0, s>>>(
+      off, skeys, n_ids, K, PW, g, ch, mu, my, sl, t.chunks.as<TileChunk>(),
+      t.multi.as<uint4>(), t.occ.as<uint32_t>(), ow);
+  GN_LAUNCH_CHECK("column chunks");
+  GN_CUDA(cudaStreamSynchronize(s));
+}
+
+// ------------------------------------------------------------------------
+// the spread
+// ------------------------------------------------------------------------
+constexpr int kSpreadWarps = 4;
+constexpr int kSpreadThreads = kSpreadWarps * 32;
+constexpr int kStageRecs = 8;  // records per pipeline stage of a warp
+constexpr int kStages = 4;
+
+// How the 32 / CL lane groups ("subs") of a warp split a column's cross
+// section: SR subs take different y rows, SX subs different runs of NX x
+// cells; every sub sees every record.  A lane holds PW x NR x NX sums.
+template <int DIM, int PW, int CL> struct Split
+{
+  using T = Tile<DIM>;
+  static constexpr int SUB = 32 / CL;
+  static constexpr int SR = SUB < T::R ? SUB : T::R;
+  static constexpr int SX = SUB / SR;
+  static constexpr int NR = T::R / SR, NX = T::X / SX;
+  static_assert(NX >= 1, "a lane holds at least one cell");
+  static constexpr int WORDS = Rec<DIM, PW>::WORDS;
+  static constexpr int stage_bytes = kStageRecs * (WORDS * 4 + CL * 8);
+  static constexpr int smem = kSpreadWarps * kStages * stage_bytes;
+  static constexpr int regs = 2 * PW * NR * NX + 2 * NX + NR * PW + 34;
+  static constexpr int MINB =
+      regs > 168 ? 2
+                 : (regs > 128 ? 3
+                               : (regs > 100 ? 4
+                                             : (regs > 80 ? 5
+                                                          : (regs > 64 ? 6
+                                                                       : 8))));
+};
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit()
+{
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+template <int N> __device__ __forceinline__ void cp_wait()
+{
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// Coils of storage per cell of the last, partial 16-coil group.
+__host__ __device__ __forceinline__ int tail_pitch(int C)
+{
+  const int r = C & 15;
+  return r == 0 ? 0 : (r <= 4 ? 4 : (r <= 8 ? 8 : 16));
+}
+
+// N consecutive floats from shared memory, in the widest loads A (alignment
+// in words) allows.
+template <int N, int A>
+__device__ __forceinline__ void lds(const float *p, float (&v)[N])
+{
+  if constexpr (A % 4 == 0 && N % 4 == 0)
+  {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i)
+    {
+      const float4 q = reinterpret_cast<const float4 *>(p)[i];
+      v[4 * i] = q.x;
+      v[4 * i + 1] = q.y;
+      v[4 * i + 2] = q.z;
+      v[4 * i + 3] = q.w;
+    }
+  }
+  else if constexpr (A % 2 == 0 && N % 2 == 0)
+  {
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i)
+    {
+      const float2 q = reinterpret_cast<const float2 *>(p)[i];
+      v[2 * i] = q.x;
+      v[2 * i + 1] = q.y;
+    }
+  }
+  else
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      v[i] = p[i];
+}
+
+// One warp per chunk and CL coils.  The chunk's records come ordered by
+// their first plane; the warp walks the planes with the sums of PW planes in
+// registers (plane p in slot p mod PW, a constant in the unrolled loop),
+// accumulates the records that start at the current plane, then writes that
+// plane and reuses its slot.  Records and k-space rows of the next
+// kStages - 1 stages are in flight (asynchronous copies into the warp's own
+// ring); the sample indices of one more stage are in registers.
+template <int DIM, int PW, int CL>
+__global__ void __launch_bounds__(kSpreadThreads, Split<DIM, PW, CL>::MINB)
+    k_tile_spread(const TileChunk *__restrict__ chunks, int n_chunks,
+                  const float *__restrict__ recs,
+                  const float2 *__restrict__ ks, int CP, int C, Geo g,
+                  float2 *__restrict__ grid, float2 *__restrict__ partial,
+                  int HP)
+{
+  using T = Tile<DIM>;
+  using S = Split<DIM, PW, CL>;
+  using R = Rec<DIM, PW>;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ci = blockIdx.x * kSpreadWarps + warp;
+  if (ci >= n_chunks)
+    return;  // warps are independent: no block barrier follows
+  // tile, begin, end, slot | p0, p1
+  const uint4 ch = __ldg(reinterpret_cast<const uint4 *>(chunks) + 2 * ci);
+  const uint4 ch2 =
+      __ldg(reinterpret_cast<const uint4 *>(chunks) + 2 * ci + 1);
+  const int group = blockIdx.y;
+  const int coil = lane % CL, sub = lane / CL;
+  const int sr = sub % S::SR, sx = sub / S::SR;
+  unsigned char *ring = smraw + (size_t)warp * kStages * S::stage_bytes;
+  const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
+  const float2 *ksg = ks + group * CL;
+  const int n = (int)(ch.z - ch.y);  // records [ch.y, ch.z)
+  const int n_st = (n + kStageRecs - 1) / kStageRecs;
+
+  auto load_idx = [&](int st) -> uint32_t {
+    const int e = st * kStageRecs + (lane & (kStageRecs - 1));
+    if (e >= n)
+      return 0u;
+    return __float_as_uint(
+        __ldg(recs + (size_t)(ch.y + (uint32_t)e) * R::WORDS + R::TW));
+  };
+  auto fill = [&](int st, uint32_t idx) {
+    const uint32_t b = ring_a + (uint32_t)(st % kStages) * S::stage_bytes;
+    const int nv = min(kStageRecs, n - st * kStageRecs);
+    // records: contiguous
+    const float *src =
+        recs + (size_t)(ch.y + (uint32_t)(st * kStageRecs)) * R::WORDS;
+    constexpr int RC = R::WORDS / 4;  // 16-byte pieces per record
+#pragma unroll
+    for (int q = 0; q < kStageRecs * RC; q += 32)
+      if (q + lane < nv * RC)
+        cp16(b + (q + lane) * 16, src + (q + lane) * 4);
+    // k-space rows of the CL coils
+    constexpr int KC = CL / 2;  // 16-byte pieces per row
+    const uint32_t kb = b + kStageRecs * R::WORDS * 4;
+#pragma unroll
+    for (int q = 0; q < kStageRecs * KC; q += 32)
+    {
+      const int e = (q + lane) / KC, part = (q + lane) % KC;
+      const uint32_t t = __shfl_sync(0xffffffffu, idx, e & (kStageRecs - 1));
+      if (e < nv)
+        cp16(kb + (q + lane) * 16, ksg + (size_t)t * CP + part * 2);
+    }
+  };
+
+  float2 acc[PW][S::NR][S::NX];
+#pragma unroll
+  for (int p = 0; p < PW; ++p)
+#pragma unroll
+    for (int r = 0; r < S::NR; ++r)
+#pragma unroll
+      for (int x = 0; x < S::NX; ++x)
+        acc[p][r][x] = make_float2(0.f, 0.f);
+
+  uint32_t idx = load_idx(0);
+#pragma unroll
+  for (int st = 0; st < kStages - 1; ++st)
+  {
+    const uint32_t nxt = load_idx(st + 1);
+    if (st < n_st)
+      fill(st, idx);
+    cp_commit();
+    idx = nxt;
+  }
+  int e = -1;              // current record
+  const float *rp = nullptr;  // its words and k-space row in the ring
+  const float2 *kp = nullptr;
+  uint32_t z0 = 0;  // its first plane + (planes << 8); ~0: no more records
+  auto advance = [&]() {
+    ++e;
+    if ((e & (kStageRecs - 1)) == 0)
+    {
+      const int st = e / kStageRecs;
+      __syncwarp();  // the previous stage is read
+      cp_wait<kStages - 2>();
+      __syncwarp();  // every lane's copies of stage st have landed
+      const uint32_t nxt = load_idx(st + kStages);
+      if (st + kStages - 1 < n_st)
+        fill(st + kStages - 1, idx);
+      cp_commit();
+      idx = nxt;
+      const unsigned char *sb = ring + (st % kStages) * S::stage_bytes;
+      rp = reinterpret_cast<const float *>(sb);
+      kp = reinterpret_cast<const float2 *>(sb + kStageRecs * R::WORDS * 4) +
+           coil;
+    }
+    else
+    {
+      rp += R::WORDS;
+      kp += CL;
+    }
+    z0 = e < n ? __float_as_uint(rp[R::TW + 1]) : ~0u;
+  };
+  advance();
+
+  int tx, ty, tz;
+  tile_of_id<DIM>(tile_dims<DIM>(g), ch.x, tx, ty, tz);
+  const int cc = group * CL + coil;  // grid coil lane
+  const int pitch = cc < (C & ~15) ? 16 : tail_pitch(C);
+  const int p0 = (int)ch2.x, p1 = (int)ch2.y;
+  // where plane 0 of the lane's cells goes, and the steps from there
+  float2 *out;
+  long long step_p, step_r;
+  int lim_p, lim_r = S::NR, lim_x = S::NX, step_x;
+  if ((int)ch.w >= 0)
+  {  // a partial column [plane][row][x][HP]
+    out = partial +
+          ((size_t)ch.w * T::CELLS + sr * S::NR * T::X + sx * S::NX) * HP +
+          cc;
+    step_p = (long long)T::R * T::X * HP;
+    step_r = (long long)T::X * HP;
+    step_x = HP;
+    lim_p = T::SEG;
+  }
+  else
+  {
+    const int x0 = tx * T::X + sx * S::NX;
+    const int y0 = DIM == 3 ? ty * T::R + sr * S::NR : ty * T::SEG;
+    const int q0 = DIM == 3 ? tz * T::SEG : 0;
+    out = grid + (size_t)(cc & ~15) * g.grid_count + (cc & 15) +
+          (((long long)q0 * g.G[1] + y0) * g.G[0] + x0) * pitch;
+    step_x = pitch;
+    step_r = (long long)g.G[0] * pitch;
+    step_p = DIM == 3 ? step_r * g.G[1] : step_r;
+    lim_p = DIM == 3 ? g.G[2] - q0 : g.G[1] - y0;
+    if (DIM == 3)
+      lim_r = g.G[1] - y0;
+    lim_x = g.G[0] - x0;
+  }
+  if (cc >= HP)
+    lim_p = 0;  // lanes beyond the grid's coils write nothing
+  out += p0 * step_p;
+
+  for (int pb = p0; pb < p1; pb += PW)
+  {
+#pragma unroll
+    for (int q = 0; q < PW; ++q)
+    {
+      const int plane = pb + q;
+      if (plane >= p1)
+        break;
+      while ((z0 & 0xffu) == (uint32_t)plane)
+      {
+        const int planes = (int)(z0 >> 8);
+        float wx[S::NX], w[S::NR][PW];
+        lds<S::NX, S::NX>(rp + sx * S::NX, wx);
+#pragma unroll
+        for (int r = 0; r < S::NR; ++r)
+          lds<PW, (R::W0 % 4 == 0 && PW % 4 == 0) ? 4 : 2>(
+              rp + R::W0 + (sr * S::NR + r) * PW, w[r]);
+        const float2 v = *kp;
+        float2 w2[S::NX];
+#pragma unroll
+        for (int x = 0; x < S::NX; ++x)
+          w2[x] = make_float2(wx[x], wx[x]);
+        advance();
+#pragma unroll
+        for (int k = 0; k < PW; ++k)
+        {
+          // the common footprints meet all but the last one or two planes
+          if (k >= (PW == 4 ? 3 : PW - 2) && k >= planes)
+            break;
+#pragma unroll
+          for (int r = 0; r < S::NR; ++r)
+          {
+            const float2 pv = make_float2(__fmul_rn(w[r][k], v.x),
+                                          __fmul_rn(w[r][k], v.y));
+#pragma unroll
+            for (int x = 0; x < S::NX; ++x)
+              acc[(q + k) % PW][r][x] =
+                  fma2(w2[x], pv, acc[(q + k) % PW][r][x]);
+          }
+        }
+      }
+      // plane done: write it, reuse its slot
+#pragma unroll
+      for (int r = 0; r < S::NR; ++r)
+      {
+#pragma unroll
+        for (int x = 0; x < S::NX; ++x)
+        {
+          if (plane < lim_p && r < lim_r && x < lim_x)
+            out[r * step_r + x * step_x] = acc[q][r][x];
+          acc[q][r][x] = make_float2(0.f, 0.f);
+        }
+      }
+      out += step_p;
+    }
+  }
+  cp_wait<0>();
+}
+
+// Columns with several chunks: their partial columns added in a fixed
+// order.  MANY false (up to kFewSlots chunks): one thread per element.  MANY
+// true: a warp finds the chunks that meet its plane (they come ordered by
+// plane), kRedLanes warps add equal runs of them and the runs' sums are
+// added in run order.
+constexpr int kRedLanes = 8;
+template <int DIM, bool MANY>
+__global__ void __launch_bounds__(32 * kRedLanes)
+    k_tile_reduce(const uint4 *__restrict__ multi,
+                  const TileChunk *__restrict__ chunks,
+                  const float2 *__restrict__ partial, int HP, int C, Geo g,
+                  float2 *__restrict__ grid)
+{
+  using T = Tile<DIM>;
+  __shared__ float2 part[kRedLanes][32];
+  const uint4 m = multi[blockIdx.x];  // column, first slot, slots, chunk
+  const int n = T::CELLS * HP;        // a multiple of 32, and per plane
+  const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+  const int i = MANY ? blockIdx.y * 32 + lane
+                     : blockIdx.y * 32 * kRedLanes + threadIdx.x;
+  if (!MANY && i >= n)
+    return;
+  const int cell = i / HP, cc = i - cell * HP;
+  const uint32_t plane = (uint32_t)(cell / (T::R * T::X));
+  const float2 *p = partial + (size_t)m.y * n + i;
+  float2 s = make_float2(0.f, 0.f);
+  if (MANY)
+  {
+    uint32_t ka = m.z, kb = 0;  // chunks [ka, kb) meet the plane
+    for (uint32_t k = 0; k < m.z; k += 32)
+    {
+      bool in = false;
+      if (k + lane < m.z)
+      {
+        const TileChunk &c = chunks[m.w + k + lane];
+        in = plane >= c.p0 && plane < c.p1;
+      }
+      const unsigned b = __ballot_sync(0xffffffffu, in);
+      if (b)
+      {
+        ka = min(ka, k + (uint32_t)__ffs(b) - 1);
+        kb = k + 32 - (uint32_t)__clz(b);
+      }
+    }
+    const uint32_t per = kb > ka ? (kb - ka + kRedLanes - 1) / kRedLanes : 0;
+    const uint32_t k0 = ka + run * per, k1 = min(kb, k0 + per);
+#pragma unroll 4
+    for (uint32_t k = k0; k < k1; ++k)
+      s = add2(s, __ldg(p + (size_t)k * n));
+    part[run][lane] = s;
+    __syncthreads();
+    if (run != 0)
+      return;
+#pragma unroll
+    for (int r = 1; r < kRedLanes; ++r)
+      s = add2(s, part[r][lane]);
+  }
+  else
+  {
+    float2 v[kFewSlots];
+#pragma unroll
+    for (uint32_t k = 0; k < kFewSlots; ++k)
+    {
+      v[k] = make_float2(0.f, 0.f);
+      if (k < m.z)
+      {
+        const TileChunk &c = chunks[m.w + k];
+        if (plane >= c.p0 && plane < c.p1)
+          v[k] = __ldg(p + (size_t)k * n);
+      }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kFewSlots; ++k)
+      s = add2(s, v[k]);
+  }
+  int tx, ty, tz;
+  tile_of_id<DIM>(tile_dims<DIM>(g), m.x, tx, ty, tz);
+  const int x = tx * T::X + cell % T::X;
+  const int y = DIM == 3 ? ty * T::R + cell / T::X % T::R
+                         : ty * T::SEG + (int)plane;
+  const int z = DIM == 3 ? tz * T::SEG + (int)plane : 0;
+  const int pitch = cc < (C & ~15) ? 16 : tail_pitch(C);
+  if (x < g.G[0] && y < g.G[1] && z < g.G[2])
+    grid[(size_t)(cc & ~15) * g.grid_count +
+         (((size_t)z * g.G[1] + y) * g.G[0] + x) * pitch + (cc & 15)] = s;
+}
+
+template <int DIM>
+int reduce_tiles(const TileTables &t, const float2 *partial, int HP, int C,
+                 const Geo &g, float2 *grid, cudaStream_t s)
+{
+  const int n = Tile<DIM>::CELLS * HP, nt = 32 * kRedLanes;
+  const uint4 *multi = t.multi.as<uint4>();
+  const TileChunk *chunks = t.chunks.as<TileChunk>();
+  if (t.n_few)
+    k_tile_reduce<DIM, false>
+        <<<dim3((unsigned)t.n_few, (unsigned)((n + nt - 1) / nt)), nt, 0, s>>>(
+            multi, chunks, partial, HP, C, g, grid);
+  if (t.n_many)
+    k_tile_reduce<DIM, true>
+        <<<dim3((unsigned)t.n_many, (unsigned)(n / 32)), nt, 0, s>>>(
+            multi + t.n_few, chunks, partial, HP, C, g, grid);
+  GN_LAUNCH_CHECK("column reduction");
+  return (t.n_few ? 1 : 0) + (t.n_many ? 1 : 0);
+}
+
+// ------------------------------------------------------------------------
+// inverse x transform of the coil-interleaved grid
+// ------------------------------------------------------------------------
+// Persistent blocks walk units of one grid row x CB coils through two
+// shared-memory buffers [x][CB]: the next unit's runs of occupied tiles are
+// copied (untiled bulk copies) while the current row is transformed in
+// place; cells of empty tiles are read as zeros.  Stage 1 runs with lanes
+// over coils (rows of CB x 8 bytes); it stores value (r, k1) of coil c at
+// lane position c ^ k1 of row r + R2 k1 -- the lanes that share a row are in
+// one warp, so a warp barrier separates the reads from the writes -- and
+// stage 2 runs with lanes over k1, which then meet different banks and write
+// consecutive x.  Bound by instruction issue (3-D 128^3, 32 coils: 1.18 ms
+// with all outputs' addresses and range tests, 0.93 ms with HALF, which also
+// drops the last butterflies' unused outputs; 4.4 GB at the HBM copy rate
+// take 0.66 ms).
+template <int L, int CB, int TX> struct XPass
+{
+  using S = fftcore::Shape<L>;
+  static constexpr int NT = CB * S::T < 32 ? 32 : CB * S::T;
+  // two row buffers; one where two do not fit
+  static constexpr int NBUF = (size_t)L * CB * 16 > 200 * 1024 ? 1 : 2;
+  static constexpr size_t smem =
+      ((size_t)NBUF * L * CB + L) * sizeof(float2) + 2 * 8 + 16;
+  static constexpr int OW = (L / TX + 31) / 32;  // occupancy words per row
+  static constexpr int WANT = L >= 512 ? 512 : 768;  // threads per SM
+  static constexpr int MINB = WANT / NT > 6 ? 6 : (NT > WANT ? 1 : WANT / NT);
+};
+
+template <int L, int CB, int TX, bool HALF>
+__global__ void __launch_bounds__(XPass<L, CB, TX>::NT,
+                                  XPass<L, CB, TX>::MINB)
+    k_tile_xpass(const float2 *__restrict__ grid,
+                 const uint32_t *__restrict__ occ, int tile_y, int tile_z,
+                 int tiles_y, Geo g, int c_first, int C,
+                 fftcore::FastDiv groups, fftcore::FastDiv rows_y,
+                 uint32_t n_units, const float2 *__restrict__ roots,
+                 float2 *__restrict__ out, tma::CopyWait cw)
+{
+  using S = fftcore::Shape<L>;
+  constexpr int OW = XPass<L, CB, TX>::OW, NBUF = XPass<L, CB, TX>::NBUF;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  float2 *bufs = reinterpret_cast<float2 *>(smraw);
+  float2 *tw = bufs + (size_t)NBUF * L * CB;
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(tw + L);
+  int &s_fail = *reinterpret_cast<int *>(mbar + 2);
+  const uint32_t bar0 = tma::smem_addr(mbar);
+  const uint32_t stride = gridDim.x;
+  const int Nx = g.N[0];
+  const long long plane = (long long)g.G[2] * g.G[1] * Nx;
+  struct Occ
+  {
+    uint32_t w[OW];
+  };
+  auto occupancy = [&](uint32_t u) {
+    Occ o;
+    const uint32_t row = groups.div(u), rz = rows_y.div(row),
+                   ry = row - rz * rows_y.d;
+    const uint32_t *p =
+        occ + ((rz >> tile_z) * (uint32_t)tiles_y + (ry >> tile_y)) * OW;
+#pragma unroll
+    for (int i = 0; i < OW; ++i)
+      o.w[i] = u < n_units ? __ldg(p + i) : 0u;
+    return o;
+  };
+  // thread 0: copy unit u's occupied cells into buffer b
+  auto issue = [&](uint32_t u, int b, const Occ &o) {
+    const uint32_t bar = bar0 + 8u * (uint32_t)b;
+    constexpr uint32_t TB = TX * CB * sizeof(float2);  // bytes per tile
+    uint32_t bytes = 0;
+#pragma unroll
+    for (int i = 0; i < OW; ++i)
+      bytes += (uint32_t)__popc(o.w[i]) * TB;
+    tma::mbar_expect_tx(bar, bytes);
+    const uint32_t row = groups.div(u), gi = u - row * groups.d;
+    const char *src = reinterpret_cast<const char *>(
+        grid + ((size_t)gi * g.grid_count + (size_t)row * L) * CB);
+    const uint32_t dst = tma::smem_addr(bufs + (size_t)b * L * CB);
+#pragma unroll
+    for (int i = 0; i < OW; ++i)
+    {
+      uint32_t m = o.w[i];
+      while (m)
+      {  // runs of set bits
+        const int lo = __ffs(m) - 1;
+        const uint32_t inv = ~(m >> lo);
+        const int len = inv ? __ffs(inv) - 1 : 32 - lo;
+        const uint32_t off = (uint32_t)(32 * i + lo) * TB;
+        tma::copy_bulk(dst + off, src + off, (uint32_t)len * TB, bar);
+        m &= len + lo >= 32 ? 0u : ~0u << (lo + len);
+      }
+    }
+  };
+  Occ cur = occupancy(blockIdx.x), nxt = occupancy(blockIdx.x + stride);
+  if (threadIdx.x == 0)
+  {
+    s_fail = 0;
+    tma::mbar_init(bar0);
+    tma::mbar_init(bar0 + 8u);
+    tma::mbar_init_fence();
+    if (blockIdx.x < n_units)
+      issue(blockIdx.x, 0, cur);
+    if (NBUF == 2 && blockIdx.x + stride < n_units)
+      issue(blockIdx.x + stride, 1, nxt);
+  }
+  fftcore::load_roots(tw, roots, L);
+  __syncthreads();
+  float2 w[fftcore::Rm<L>::V / 2];
+  fftcore::load_reg_roots<L>(w, tw);
+  // FFT output k holds image x = (k - crop - floor(G/2)) mod G when < N;
+  // HALF: osf 2 (crop L / 4), x = k + L / 4 mod L
+  int add = (-(g.crop[0] + g.shift_inv[0])) % L;
+  add += add < 0 ? L : 0;
+  uint32_t it = 0;
+  for (uint32_t u = blockIdx.x; u < n_units; u += stride, ++it)
+  {
+    const int b = NBUF == 2 ? (int)(it & 1) : 0;
+    const uint32_t phase = (NBUF == 2 ? it >> 1 : it) & 1u;
+    const Occ nn = occupancy(u + 2 * stride);
+    const uint32_t row = groups.div(u), gi = u - row * groups.d;
+    const uint32_t rz = rows_y.div(row);
+    int y = (int)(row - rz * rows_y.d) - g.shift_inv[1];
+    int z = (int)rz - g.shift_inv[2];
+    y += y < 0 ? g.G[1] : 0;
+    z += z < 0 ? g.G[2] : 0;
+    float2 *buf = bufs + (size_t)b * L * CB;
+    if (threadIdx.x == 0 &&
+        !tma::mbar_wait_bounded(bar0 + 8u * (uint32_t)b, phase, cw.polls))
+      s_fail = 1;
+    __syncthreads();
+    if (s_fail)
+    {  // a copy did not complete: report it and give the copies in flight
+       // a bounded wait before the shared memory is released
+      if (threadIdx.x == 0)
+      {
+        atomicExch(cw.err, 1);
+        tma::mbar_wait_bounded(bar0 + 8u * (uint32_t)b, phase);
+        if (NBUF == 2 && u + stride < n_units)
+          tma::mbar_wait_bounded(bar0 + 8u * (uint32_t)(b ^ 1),
+                                 ((it + 1) >> 1) & 1u);
+      }
+      return;
+    }
+    {
+      const int c = threadIdx.x % CB, r = threadIdx.x / CB;
+      float2 a[S::R1];
+      if (r < S::R2)
+      {
+        // FFT input n holds cell (n + L / 2) mod L, of the same residue
+        // class mod R2
+#pragma unroll
+        for (int j = 0; j < S::R1; ++j)
+        {
+          const int jj = (j + S::R1 / 2) % S::R1;
+          // tile of cell r + R2 jj; with R2 a multiple of TX (or TX of R2)
+          // the word and most of the shift are constants
+          const int tb = S::R2 % TX == 0 ? S::R2 / TX * jj : 0;
+          const int ti = S::R2 % TX == 0 ? r / TX : (r + S::R2 * jj) / TX;
+          const bool on =
+              (cur.w[(S::R2 % TX == 0 ? tb : S::R2 * jj / TX) >> 5] >>
+               (ti & 31)) &
+              (1u << (tb & 31));
+          a[j] = on ? buf[(r + S::R2 * jj) * CB + c] : make_float2(0.f, 0.f);
+        }
+      }
+      __syncwarp();
+      if (r < S::R2)
+      {
+        fftcore::reg_fft<S::R1, fftcore::Rm<L>::V, true>(a, w);
+#pragma unroll
+        for (int k1 = 0; k1 < S::R1; ++k1)
+        {
+          float2 v = a[k1];
+          if (k1 != 0)
+          {
+            float2 t = tw[r * k1];
+            t.y = -t.y;
+            v = cmul(v, t);
+          }
+          buf[(r + S::R2 * k1) * CB + (c ^ (k1 & (CB - 1)))] = v;
+        }
+      }
+    }
+    __syncthreads();
+    const int k1 = threadIdx.x % S::T, cl = threadIdx.x / S::T;
+    const int c = c_first + (int)gi * CB + cl;
+    float2 bb[S::R2];
+    const bool live = k1 < S::R1 && cl < CB && c < C;
+    if (live)
+    {
+#pragma unroll
+      for (int r = 0; r < S::R2; ++r)
+        bb[r] = buf[(r + S::R2 * k1) * CB + (cl ^ (k1 & (CB - 1)))];
+    }
+    tma::fence_proxy_async();  // the in-place writes before the refill
+    __syncthreads();           // buffer b is free
+    if (threadIdx.x == 0 && u + NBUF * stride < n_units)
+      issue(u + NBUF * stride, b, NBUF == 2 ? nn : nxt);
+    if (live)
+    {
+      fftcore::reg_fft<S::R2, fftcore::Rm<L>::V, true>(bb, w);
+      float2 *o = out + (long long)c * plane +
+                  ((long long)z * g.G[1] + y) * Nx;
+      if constexpr (HALF)
+      {  // N = G / 2: the outputs k < L / 4 and k >= 3 L / 4, constant steps
+        o += k1 + L / 4;
+#pragma unroll
+        for (int k2 = 0; k2 < S::R2 / 4; ++k2)
+        {
+          o[S::R1 * k2] = bb[k2];
+          o[S::R1 * (k2 - S::R2 / 4)] = bb[k2 + 3 * S::R2 / 4];
+        }
+      }
+      else
+      {
+#pragma unroll
+        for (int k2 = 0; k2 < S::R2; ++k2)
+        {
+          const int x = (k1 + S::R1 * k2 + add) & (L - 1);
+          if (x < Nx)
+            o[x] = bb[k2];
+        }
+      }
+    }
+    cur = nxt;
+    nxt = nn;
+  }
+}
+
+template <class K> void set_smem(K k, size_t bytes)
+{
+  if (bytes > 48 * 1024)
+    GN_CUDA(cudaFuncSetAttribute(
+        k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
+template <int DIM, int PW, int CL>
+void spread(const TileTables &t, const float2 *ks, int CP, int C,
+            const Geo &g, float2 *grid, float2 *partial, cudaStream_t s)
+{
+  using S = Split<DIM, PW, CL>;
+  auto k = k_tile_spread<DIM, PW, CL>;
+  set_smem(k, S::smem);
+  const dim3 grd((unsigned)((t.n_chunks + kSpreadWarps - 1) / kSpreadWarps),
+                 (unsigned)(CP / CL));
+  k<<<grd, kSpreadThreads, S::smem, s>>>(t.chunks.as<TileChunk>(), t.n_chunks,
+                                         t.recs.as<float>(), ks, CP, C, g,
+                                         grid, partial, tile_grid_pitch(C));
+  GN_LAUNCH_CHECK("column spread");
+}
+
+// Planes a footprint (at most kw + 1 cells) can meet, as instantiated.
+template <class F> void with_planes(const Geo &g, F f)
+{
+  if (g.kw <= 3)
+    f(std::integral_constant<int, 4>());
+  else if (g.kw <= 5)
+    f(std::integral_constant<int, 6>());
+  else
+    f(std::integral_constant<int, 8>());
+}
+}  // namespace
+
+bool tile_spread_supported(const Geo &g)
+{
+  for (int a = 0; a < g.dim; ++a)
+    if (g.G[a] < (a == 2 ? Tile<3>::SEG : 8) + kSlots)
+      return false;
+  return true;
+}
+
+void build_tile_tables(const float *traj_sorted, const uint32_t *sector_sorted,
+                       uint32_t M, const Geo &g, const float *lut,
+                       TileTables &t, BuildWork &work, cudaStream_t s)
+{
+  if (!M)
+    return;
+  with_planes(g, [&](auto pw) {
+    constexpr int PW = decltype(pw)::value;
+    if (g.dim == 3)
+      build_tables<3, PW>(traj_sorted, sector_sorted, M, g, lut, t, work,
+                          s);
+    else
+      build_tables<2, PW>(traj_sorted, sector_sorted, M, g, lut, t, work,
+                          s);
+  });
+}
+
+int tile_coil_lanes(int CP)
+{
+  for (int cl = 32; cl >= 4; cl >>= 1)
+    if (CP % cl == 0)
+      return cl;
+  return 0;
+}
+
+int tile_grid_pitch(int C) { return (C & ~15) + tail_pitch(C); }
+
+size_t tile_partial_elems(const TileTables &t, const Geo &g, int C)
+{
+  const size_t cells = g.dim == 3 ? Tile<3>::CELLS : Tile<2>::CELLS;
+  return (size_t)t.n_slots * cells * tile_grid_pitch(C);
+}
+
+int launch_tile_spread(const TileTables &t, const float2 *ks, int CP,
+                       const Geo &g, int C, float2 *grid, float2 *partial,
+                       cudaStream_t s)
+{
+  const int HP = tile_grid_pitch(C);
+  with_planes(g, [&](auto pw) {
+    constexpr int PW = decltype(pw)::value;
+    auto go = [&](auto clc) {
+      constexpr int CL = decltype(clc)::value;
+      if (g.dim == 3)
+        spread<3, PW, CL>(t, ks, CP, C, g, grid, partial, s);
+      else
+        spread<2, PW, CL>(t, ks, CP, C, g, grid, partial, s);
+    };
+    switch (tile_coil_lanes(CP))
+    {
+    case 32: go(std::integral_constant<int, 32>()); break;
+    case 16: go(std::integral_constant<int, 16>()); break;
+    case 8: go(std::integral_constant<int, 8>()); break;
+    default: go(std::integral_constant<int, 4>()); break;
+    }
+  });
+  return 1 + (g.dim == 3 ? reduce_tiles<3>(t, partial, HP, C, g, grid, s)
+                         : reduce_tiles<2>(t, partial, HP, C, g, grid, s));
+}
+
+bool tile_xpass_supported(const Geo &g)
+{
+  const int L = g.G[0];
+  return L >= 16 && L <= 1024 && (L & (L - 1)) == 0;
+}
+
+void launch_tile_xpass(const TileTables &t, const float2 *grid,
+                       const Geo &g, int C, const float2 *roots_x,
+                       float2 *out, tma::CopyWait cw, cudaStream_t s)
+{
+  // log2 of the columns' extents (powers of two)
+  const int ty = fftcore::ilog2(g.dim == 3 ? Tile<3>::Y : Tile<2>::Y);
+  const int tz = fftcore::ilog2(g.dim == 3 ? Tile<3>::Z : Tile<2>::Z);
+  const int tiles_y = (g.G[1] + (1 << ty) - 1) >> ty;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // groups of CB coils from coil c_first on
+  auto go = [&](auto lc, auto cbc, int c_first, int groups) {
+    constexpr int L = decltype(lc)::value, CB = decltype(cbc)::value;
+    auto launch = [&](auto txc, auto half) {
+      constexpr int TX = decltype(txc)::value;
+      using X = XPass<L, CB, TX>;
+      auto k = k_tile_xpass<L, CB, TX, decltype(half)::value>;
+      set_smem(k, X::smem);
+      int per_sm = 1;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, X::NT,
+                                                        X::smem) !=
+              cudaSuccess ||
+          per_sm < 1)
+        per_sm = 1;
+      const uint32_t units = (uint32_t)g.G[1] * g.G[2] * groups;
+      const uint32_t cap = (uint32_t)(per_sm * sms);
+      k<<<units < cap ? units : cap, X::NT, X::smem, s>>>(
+          grid + (size_t)c_first * g.grid_count, t.occ.as<uint32_t>(), ty, tz,
+          tiles_y, g, c_first, C, fftcore::FastDiv((uint32_t)groups),
+          fftcore::FastDiv((uint32_t)g.G[1]), units, roots_x, out, cw);
+      GN_LAUNCH_CHECK("inverse x transform of the column grid");
+    };
+    const bool half = g.N[0] == L / 2 && g.crop[0] == L / 4;
+    auto pick = [&](auto txc) {
+      if (half)
+        launch(txc, std::true_type());
+      else
+        launch(txc, std::false_type());
+    };
+    if (g.dim == 3)
+      pick(std::integral_constant<int, Tile<3>::X>());
+    else
+      pick(std::integral_constant<int, Tile<2>::X>());
+  };
+  auto with = [&](auto lc) {
+    const int full = C / 16, tail = tail_pitch(C);
+    if (full)
+      go(lc, std::integral_constant<int, 16>(), 0, full);
+    if (tail == 16)
+      go(lc, std::integral_constant<int, 16>(), 16 * full, 1);
+    else if (tail == 8)
+      go(lc, std::integral_constant<int, 8>(), 16 * full, 1);
+    else if (tail == 4)
+      go(lc, std::integral_constant<int, 4>(), 16 * full, 1);
+  };
+  switch (g.G[0])
+  {
+  case 16: with(std::integral_constant<int, 16>()); break;
+  case 32: with(std::integral_constant<int, 32>()); break;
+  case 64: with(std::integral_constant<int, 64>()); break;
+  case 128: with(std::integral_constant<int, 128>()); break;
+  case 256: with(std::integral_constant<int, 256>()); break;
+  case 512: with(std::integral_constant<int, 512>()); break;
+  case 1024: with(std::integral_constant<int, 1024>()); break;
+  default: throw Error(kInternal, "no x transform for this row length");
+  }
+}
+
+}  // namespace gnufft

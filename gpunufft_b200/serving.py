@@ -72,9 +72,10 @@ def plan_table_bytes(req: Request) -> int:
     trajectory before any call: sorted trajectory, indices (sorted order,
     sector, inverse), density weights, the interpolation matrix (row offsets
     per grid cell, at most (kw + 1)^d entries of 8 bytes per sample), the
-    forward work items, their lane order (3-D), column ranges and the list
-    of column tiles holding one, deapodization, the lookup table and the
-    maps the request sets."""
+    records of the column spread (at most a column more per axis than a
+    footprint fills), the forward work items, their lane order (3-D),
+    column ranges and the list of column tiles holding one, deapodization,
+    the lookup table and the maps the request sets."""
     dims = [v for v in req.img_dims if v]
     dim = len(dims)
     M = req.traj.shape[1]
@@ -90,6 +91,17 @@ def plan_table_bytes(req: Request) -> int:
                                        for g in grid])) + 1)
     b += 8 * grid[0] * grid[1] + 4 * (grid[0] * grid[1] // 8 + 1)
     b += 4 * N + 4 * 4096 + 8 * Cn * N
+    cells = req.kernel_width + 1
+    planes = 4 if cells <= 4 else (6 if cells <= 6 else 8)
+    if dim == 3:  # columns of 4 x 2 x 16 cells
+        rec = M * (((cells + 2) // 4 + 1) * (cells // 2 + 1) *
+                   ((cells + 14) // 16 + 1))
+        words, cols = 8 + 2 * planes, -(-grid[0] // 4) * -(-grid[1] // 2) * (
+            -(-grid[2] // 16))
+    else:         # columns of 8 x 8 cells
+        rec = M * ((cells + 6) // 8 + 1) ** 2
+        words, cols = 12 + planes, -(-grid[0] // 8) * -(-grid[1] // 8)
+    b += 4 * words * rec + 32 * (cols + rec // 128 + 1) + 16 * cols
     return int(b)
 
 

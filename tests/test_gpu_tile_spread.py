@@ -1,0 +1,82 @@
+"""The column spread (register columns, coil-interleaved grid, separate x
+transform) against the CSR product with cuFFT, coil by coil (plain plans)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+import gpunufft_b200 as G  # noqa: E402
+
+
+def _traj(dim, M, rng, dense):
+    """Random samples over the whole range (wrapped footprints); ``dense``
+    puts most of them into a few cells (columns of many chunks)."""
+    t = rng.uniform(-0.5, 0.5, (dim, M))
+    if dense:
+        n = M * 3 // 4
+        t[:, :n] = rng.uniform(-0.03, 0.03, (dim, n))
+        t[:, :8] = -0.5
+    return np.clip(t, -0.5, np.nextafter(np.float32(0.5), 0)).astype(
+        np.float32)
+
+
+# image, osf, kernel width, coils, samples, dense, operator type, maps: 4, 6
+# and 8 planes per footprint; 4, 8, 16 and 32 coil lanes, tails of 4, 8 and
+# 16 coils; the shortest grids (32) and longest rows (1024) it takes; osf
+# with and without the N = G / 2 shortcut
+CASES = [
+    ((16, 16, 16), 2.0, 3, 32, 30000, True, G.BALANCED, True),
+    ((16, 32, 64), 2.0, 3, 5, 150000, False, G.BALANCED, False),
+    ((20, 40, 20), 1.6, 3, 11, 70000, True, G.DEFAULT, False),
+    ((32, 32, 32), 2.0, 3, 20, 30000, False, G.BALANCED_TEXTURE, True),
+    ((16, 16, 16), 2.0, 5, 3, 60000, True, G.BALANCED, False),
+    ((16, 16, 32), 2.0, 7, 16, 9000, False, G.BALANCED, True),
+    ((32, 16, 16), 2.0, 4, 49, 12000, True, G.BALANCED, False),
+    ((64, 64), 2.0, 3, 17, 40000, True, G.BALANCED, True),
+    ((40, 80), 1.6, 3, 33, 30000, False, G.TEXTURE, False),
+    ((128, 16), 2.0, 5, 3, 60000, True, G.BALANCED, False),
+    ((16, 128), 2.0, 7, 12, 20000, False, G.BALANCED, True),
+    ((512, 32), 2.0, 3, 3, 120000, False, G.BALANCED, False),
+    ((512, 16), 2.0, 2, 24, 40000, True, G.BALANCED, True),
+]
+
+
+@pytest.mark.parametrize("dims,osf,kw,C,M,dense,op,maps", CASES)
+def test_column_spread_matches_csr_product(dims, osf, kw, C, M, dense, op,
+                                           maps):
+    rng = np.random.default_rng(7)
+    shape = tuple(dims[::-1])
+    traj = _traj(len(dims), M, rng, dense)
+    dens = rng.uniform(0.1, 1.0, M).astype(np.float32)
+    sens = None
+    if maps:
+        sens = (rng.standard_normal((C,) + shape) + 1j * rng.standard_normal(
+            (C,) + shape)).astype(np.complex64)
+    k = (rng.standard_normal((C, M)) + 1j * rng.standard_normal(
+        (C, M))).astype(np.complex64)
+    kt = torch.from_numpy(k).cuda()
+    args = (traj, dims, kw, 8, osf, dens, sens, op)
+    p = G.Plan(*args)
+    ref = G.Plan(*args, plain=True)
+    a = p.adjoint(kt)
+    b = p.adjoint(kt)
+    launches = p.stage_times()["launches"]
+    want = ref.adjoint(kt)
+    # gather, spread, x pass and the other axes, with the reductions of
+    # columns of several chunks; the CSR path has one launch less
+    assert launches >= 2 + len(dims)
+    assert torch.equal(a, b), "the summation order is fixed"
+    err = float(torch.linalg.vector_norm(a - want) /
+                torch.linalg.vector_norm(want))
+    # both sum 32-bit products in different orders: rounding 6e-8 per step
+    # over trees of up to a few thousand samples and 30 butterfly stages
+    assert err < 2e-6, err
+    if maps:  # the FFT stage keeps the coils apart
+        a = p.adjoint(kt, G.FFT)
+        want = ref.adjoint(kt, G.FFT)
+        err = float(torch.linalg.vector_norm(a - want) /
+                    torch.linalg.vector_norm(want))
+        assert err < 2e-6, err
+    p.close()
+    ref.close()
