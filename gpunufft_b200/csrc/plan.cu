@@ -638,6 +638,12 @@ bool tile_path(const gnufft_plan &p, uint32_t C)
   return C > 8 && work >= 6e6;
 }
 
+// The forward's grid holds coil pairs interleaved (3-D separable path).
+bool paired_grid(const gnufft_plan &p)
+{
+  return p.pruned && p.copy_err_d && forward_pairs(p.g, p.fwd_tile_coils);
+}
+
 // Complex elements of the adjoint's x-transformed rows.
 size_t xrows_elems(const Geo &g, uint32_t C)
 {
@@ -777,8 +783,7 @@ void forward_batched(gnufft_plan &p, const float2 *img, float2 *k, uint32_t C,
   }
   const bool dens_est = stage == GNUFFT_DENSITY_ESTIMATION;
   // 3-D pruned path: the grid holds coil pairs interleaved
-  const bool paired = p.pruned && !dens_est && p.copy_err_d &&
-                      forward_pairs(g, p.fwd_tile_coils);
+  const bool paired = !dens_est && paired_grid(p);
   p.grid.ensure((size_t)(paired ? (C + 1) / 2 * 2 : C) * g.grid_count *
                 sizeof(float2));
   float2 *grid = p.grid.as<float2>();
@@ -884,29 +889,83 @@ void traj_grad(gnufft_plan &p, const float2 *img, const float2 *u, uint32_t C,
   p.launches += 3;
 }
 
-// Device scratch the plan's buffers grow to for calls with C coils
-// (forward and adjoint share them): the sorted k-space lanes, the grid and
-// the transform passes' buffers (cuFFT's work area counted as one grid).
-size_t call_scratch_bytes(const gnufft_plan &p, uint32_t C)
+// Complex elements that one call with C coils needs of each scratch buffer.
+struct ScratchNeeds
+{
+  size_t ks = 0, grid = 0, fft_a = 0, fft_b = 0, tile_part = 0;
+  void merge(const ScratchNeeds &o)
+  {
+    ks = std::max(ks, o.ks);
+    grid = std::max(grid, o.grid);
+    fft_a = std::max(fft_a, o.fft_a);
+    fft_b = std::max(fft_b, o.fft_b);
+    tile_part = std::max(tile_part, o.tile_part);
+  }
+  size_t bytes() const
+  {
+    return (ks + grid + fft_a + fft_b + tile_part) * sizeof(float2);
+  }
+};
+
+ScratchNeeds forward_needs(const gnufft_plan &p, uint32_t C)
+{
+  ScratchNeeds n;
+  n.grid = (size_t)(paired_grid(p) ? (C + 1) / 2 * 2 : C) *
+           (size_t)p.g.grid_count;
+  if (p.pruned)
+  {
+    n.fft_a = pruned_scratch_a(p.g, (int)C);
+    n.fft_b = std::max(pruned_scratch_b(p.g, (int)C),
+                       pruned_scratch_xfirst(p.g, (int)C));
+  }
+  return n;
+}
+
+ScratchNeeds adjoint_needs(const gnufft_plan &p, uint32_t C)
 {
   const Geo &g = p.g;
-  const size_t G = (size_t)g.grid_count, f2 = sizeof(float2);
   const size_t cg = (size_t)spmm_coil_group((int)C);
-  const size_t CP = (C + cg - 1) / cg * cg;
+  ScratchNeeds n;
+  n.ks = (size_t)p.M * ((C + cg - 1) / cg * cg);
   const bool tiled = tile_path(p, C);
-  const size_t pitch = std::max<size_t>(
-      (C + 1) / 2 * 2, tiled ? (size_t)tile_grid_pitch((int)C) : 0);
-  size_t b = (size_t)p.M * CP * f2 + pitch * G * f2;
+  n.grid = (size_t)(tiled ? tile_grid_pitch((int)C) : (int)C) *
+           (size_t)g.grid_count;
   if (p.pruned)
-    b += (pruned_scratch_a(g, (int)C) +
-          std::max({pruned_scratch_b(g, (int)C),
-                    pruned_scratch_xfirst(g, (int)C),
-                    tiled ? xrows_elems(g, C) : (size_t)0}) +
-          (tiled ? tile_partial_elems(p.tiles, g, (int)C) : 0)) *
-         f2;
-  else
-    b += (size_t)C * G * f2;
+  {
+    n.fft_a = pruned_scratch_a(g, (int)C);
+    n.fft_b = std::max(pruned_scratch_b(g, (int)C),
+                       pruned_scratch_xfirst(g, (int)C));
+  }
+  if (tiled)
+  {
+    n.fft_b = std::max(n.fft_b, xrows_elems(g, C));
+    n.tile_part = tile_partial_elems(p.tiles, g, (int)C);
+  }
+  return n;
+}
+
+// Device scratch the plan's buffers grow to for calls with C coils
+// (forward and adjoint share them), cuFFT's work area counted as one grid.
+size_t call_scratch_bytes(const gnufft_plan &p, uint32_t C)
+{
+  ScratchNeeds n = forward_needs(p, C);
+  n.merge(adjoint_needs(p, C));
+  size_t b = n.bytes();
+  if (!p.pruned)
+    b += (size_t)C * p.g.grid_count * sizeof(float2);
   return b;
+}
+
+// The plan's buffers (and cuFFT plan) hold all that a call needs: it
+// allocates nothing.
+bool scratch_held(const gnufft_plan &p, const ScratchNeeds &n, uint32_t C)
+{
+  auto has = [](const DeviceBuffer &b, size_t elems) {
+    return b.bytes() >= elems * sizeof(float2);
+  };
+  return has(p.ks, n.ks) && has(p.grid, n.grid) && has(p.fft_a, n.fft_a) &&
+         has(p.fft_b, n.fft_b) && has(p.tile_part, n.tile_part) &&
+         (p.pruned || p.fft.count((int)C) != 0);
 }
 
 size_t held_scratch_bytes(const gnufft_plan &p)
@@ -920,11 +979,18 @@ size_t held_scratch_bytes(const gnufft_plan &p)
 // already, minus a margin) -- the upstream's concurrent coil count
 // (computePossibleConcurrentCoilCount, gpuNUFFT_operator.cpp:327-368),
 // for 2-D and 3-D alike.  At least one coil.
-uint32_t coils_per_pass(const gnufft_plan &p, uint32_t C)
+// A call whose scratch the plan holds already allocates nothing and runs in
+// one pass without asking for the free memory, which costs more host time
+// than the rest of a small call (a call of 2-D 128^2, one coil: 106 us with
+// the query, 37 us without).
+uint32_t coils_per_pass(const gnufft_plan &p, uint32_t C,
+                        const ScratchNeeds &needs)
 {
   size_t limit = p.mem_limit;
   if (!limit)
   {
+    if (scratch_held(p, needs, C))
+      return C;
     size_t free_b = 0, total_b = 0;
     GN_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t margin = (size_t)256 << 20;
@@ -951,7 +1017,7 @@ uint32_t coils_per_pass(const gnufft_plan &p, uint32_t C)
 void adjoint_chunked(gnufft_plan &p, const float2 *k, float2 *img,
                      uint32_t C, int stage, cudaStream_t s)
 {
-  const uint32_t step = coils_per_pass(p, C);
+  const uint32_t step = coils_per_pass(p, C, adjoint_needs(p, C));
   const float2 *sens = p.sens.as<float2>();
   const bool combine = stage == GNUFFT_DEAPODIZATION && sens;
   const bool conv = stage == GNUFFT_CONVOLUTION ||
@@ -971,7 +1037,7 @@ void adjoint_chunked(gnufft_plan &p, const float2 *k, float2 *img,
 void forward_chunked(gnufft_plan &p, const float2 *img, float2 *k,
                      uint32_t C, int stage, cudaStream_t s)
 {
-  const uint32_t step = coils_per_pass(p, C);
+  const uint32_t step = coils_per_pass(p, C, forward_needs(p, C));
   const float2 *sens = p.sens.as<float2>();
   const size_t N = (size_t)p.g.img_count;
   for (uint32_t c0 = 0; c0 < C; c0 += step)
