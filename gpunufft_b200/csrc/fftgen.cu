@@ -1,0 +1,615 @@
+// Pruned transform passes for general line lengths (see fftgen.cuh).
+//
+// A line is two (L = R0 R2) or three (L = R0 R1 R2) register DFT stages with
+// exchanges through shared memory; the lengths are run-time values and each
+// stage switches over the radices.  The inverse transform swaps the parts on
+// the way in and out.
+//
+// Bound by instruction issue and the latency of short blocks.  3-D 96^3 on
+// 192^3, 16 coils on a B200: forward x / y / z 0.15 / 0.18 / 0.33 ms where
+// cuFFT and the padding pass took 1.30 ms over the whole zero-padded grid;
+// adjoint x / y / z with the coil sum 0.36 / 0.18 / 0.15 ms against 1.12 ms.
+#include "fftgen.cuh"
+
+#include <algorithm>
+
+#include "cplx.cuh"
+#include "devutil.hpp"
+#include "fftcore.cuh"
+#include "regdft.cuh"
+
+namespace gnufft
+{
+namespace
+{
+constexpr int kLanes = 16;     // lines per block
+constexpr int kMaxRadix = 16;  // a thread's values of one stage
+
+// The factors of a line, R[0] first; R[1] 1: two stages.  `threads` per
+// line.
+struct Factors
+{
+  int L, R[3], threads;
+};
+
+constexpr int kMaxThreads = kLanes * kMaxRadix;
+constexpr int kMinBlocks = 4;  // 64 registers: a few spilled words in the
+                               // largest radices, a third more lines in flight
+
+// f(float2 (&)[R]) for a run-time radix R
+template <class F> __device__ __forceinline__ void with_radix(int R, F f)
+{
+#define GN_R(V)                                                                \
+  case V:                                                                      \
+  {                                                                            \
+    float2 a[V];                                                               \
+    f(a);                                                                      \
+    break;                                                                     \
+  }
+  switch (R)
+  {
+    GN_R(2) GN_R(3) GN_R(4) GN_R(5) GN_R(6) GN_R(7) GN_R(8) GN_R(9) GN_R(10)
+    GN_R(11) GN_R(12) GN_R(13) GN_R(14) GN_R(15) GN_R(16)
+  }
+#undef GN_R
+}
+
+template <int R>
+__device__ __forceinline__ void transform(float2 (&a)[R])
+{
+  regdft::Dft<R>::run(a);
+}
+
+// (v.y, v.x) when SWAP: the inverse transform by a forward one
+template <bool SWAP> __device__ __forceinline__ float2 part_swap(float2 v)
+{
+  return SWAP ? make_float2(v.y, v.x) : v;
+}
+
+// A line's stages (line lane cl, thread-in-line lt).  Residue r of stage 0
+// (r < M = L / R0) takes inputs r + M j -- load(r, M, a) -- and leaves value
+// k0 in row r + M k0 of buf; the M rows of each k0 are then a transform of
+// their own, of R1 x R2 points, whose stage 1 works in place.  Item
+// q = k0 R1 + k1 of the last stage reads rows q R2 + r and gives outputs
+// k0 + R0 (k1 + R1 k2): store(k0 + R0 k1, R0 R1, a).  A barrier precedes
+// each later stage.
+template <int PITCH, class Load, class Store>
+__device__ __forceinline__ void line_dft(const Factors &f, float2 *buf, int cl,
+                                         int lt, bool on, const float2 *tw,
+                                         Load load, Store store)
+{
+  const int M = f.L / f.R[0];
+  if (on)
+    for (int r = lt; r < M; r += f.threads)
+      with_radix(f.R[0], [&](auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        load(r, M, a);
+        transform(a);
+        float2 *q = buf + r * PITCH + cl;
+        q[0] = a[0];
+        const int step = M * PITCH;
+#pragma unroll
+        for (int k = 1; k < R; ++k)
+          q[k * step] = cmul(a[k], tw[k * r]);
+      });
+  __syncthreads();
+  if (f.R[1] > 1)
+  {
+    if (on)
+      for (int it = lt; it < f.R[0] * f.R[2]; it += f.threads)
+      {
+        const int k0 = it / f.R[2], r = it - k0 * f.R[2];
+        float2 *q = buf + (k0 * M + r) * PITCH + cl;
+        const int step = f.R[2] * PITCH, tr = r * f.R[0];
+        with_radix(f.R[1], [&](auto &a) {
+          constexpr int R = sizeof(a) / sizeof(a[0]);
+#pragma unroll
+          for (int j = 0; j < R; ++j)
+            a[j] = q[j * step];
+          transform(a);
+          q[0] = a[0];
+#pragma unroll
+          for (int k = 1; k < R; ++k)
+            q[k * step] = cmul(a[k], tw[k * tr]);
+        });
+      }
+    __syncthreads();
+  }
+  if (on)
+    for (int it = lt; it < f.R[0] * f.R[1]; it += f.threads)
+    {
+      const int k0 = it / f.R[1];
+      const int k = k0 + f.R[0] * (it - k0 * f.R[1]);
+      const float2 *q = buf + it * f.R[2] * PITCH + cl;
+      with_radix(f.R[2], [&](auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+          a[j] = q[j * PITCH];
+        transform(a);
+        store(k, f.R[0] * f.R[1], a);
+      });
+    }
+}
+
+// --------------------------------------------------------------------------
+// column pass
+// --------------------------------------------------------------------------
+template <bool INV, bool PAIRED>
+__global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
+    k_gen_cols(const float2 *__restrict__ src, float2 *__restrict__ dst,
+               Factors f, long long ncols, int src_rows, int dst_rows,
+               long long planes, int in_add, int in_count, int out_add,
+               int out_count, const float2 *__restrict__ roots,
+               const uint2 *__restrict__ colrange,
+               const uint32_t *__restrict__ tiles)
+{
+  extern __shared__ float2 sm[];
+  float2 *tw = sm, *buf = sm + f.L;
+  fftcore::load_roots(tw, roots, f.L);
+  const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
+  long long plane, col;
+  if (PAIRED)
+  {  // 8 columns of both coils of a pair, the coils alternating per column
+     // so that a half warp stores whole pairs
+    const long long ct = tiles ? __ldg(tiles + blockIdx.x) : blockIdx.x;
+    col = ct * (kLanes / 2) + cl / 2;
+    plane = 2LL * blockIdx.y + cl % 2;
+  }
+  else
+  {
+    col = (long long)blockIdx.x * kLanes + cl;
+    plane = blockIdx.y;
+  }
+  bool on = col < ncols && plane < planes;
+  uint32_t lo = 0, span = (uint32_t)out_count;  // output rows lo + [0, span)
+  if (colrange && on)
+  {
+    const uint2 cr = __ldg(colrange + col);
+    on = cr.x <= cr.y && cr.x < span;
+    lo = cr.x;
+    span = min(cr.y + 1, span) - lo;
+  }
+  __syncthreads();
+  const float2 *sp = src + plane * src_rows * ncols + col;
+  const long long psz = (long long)dst_rows * ncols;
+  float2 *dp = PAIRED ? dst + ((plane >> 1) * psz + col) * 2 + (plane & 1)
+                      : dst + plane * psz + col;
+  const uint32_t is = (uint32_t)ncols, os = PAIRED ? 2 * is : is;
+  line_dft<kLanes>(
+      f, buf, cl, lt, on, tw,
+      [&](int r, int step, auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        r += in_add;
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+          int row = r + j * step;
+          row -= row >= f.L ? f.L : 0;
+          a[j] = part_swap<INV>(row < in_count
+                                    ? __ldg(sp + (size_t)(uint32_t)row * is)
+                                    : make_float2(0.f, 0.f));
+        }
+      },
+      [&](int k, int step, auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        k += out_add;
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+          int row = k + j * step;
+          row -= row >= f.L ? f.L : 0;
+          if ((uint32_t)row - lo < span)
+            dp[(size_t)(uint32_t)row * os] = part_swap<INV>(a[j]);
+        }
+      });
+}
+
+// --------------------------------------------------------------------------
+// last adjoint pass
+// --------------------------------------------------------------------------
+__global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
+    k_gen_cols_sum(const float2 *__restrict__ src, Factors f, long long ncols,
+                   long long coil_stride, const float *__restrict__ deapo,
+                   const float2 *__restrict__ sens, int n_out, long long N,
+                   int C, int cpb, int out_add, float scale, int stage_out,
+                   int accumulate, const float2 *__restrict__ roots,
+                   float2 *__restrict__ out, float2 *__restrict__ partial)
+{
+  extern __shared__ float2 sm[];
+  float2 *tw = sm, *buf = sm + f.L;
+  const bool sum = sens != nullptr && stage_out == 2;
+  float2 *acc = buf + f.L * kLanes;  // [n_out][kLanes], with `sum`
+  fftcore::load_roots(tw, roots, f.L);
+  const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
+  const long long col = (long long)blockIdx.x * kLanes + cl;
+  const bool on = col < ncols;
+  const int c0 = blockIdx.y * cpb, c1 = min(C, c0 + cpb);
+  const uint32_t is = (uint32_t)ncols;
+  __syncthreads();
+  for (int c = c0; c < c1; ++c)
+  {
+    const float2 *sp = src + c * coil_stride + col;
+    line_dft<kLanes>(
+        f, buf, cl, lt, on, tw,
+        [&](int r, int step, auto &a) {
+          constexpr int R = sizeof(a) / sizeof(a[0]);
+#pragma unroll
+          for (int j = 0; j < R; ++j)
+            a[j] = part_swap<true>(
+                __ldg(sp + (size_t)(uint32_t)(r + j * step) * is));
+        },
+        [&](int k, int step, auto &a) {
+          constexpr int R = sizeof(a) / sizeof(a[0]);
+          k += out_add;
+#pragma unroll
+          for (int j = 0; j < R; ++j)
+          {
+            int n = k + j * step;
+            n -= n >= f.L ? f.L : 0;
+            if (n >= n_out)
+              continue;
+            const size_t px = (size_t)(uint32_t)n * is + (size_t)col;
+            // crop -> FFT scaling -> deapodization -> conj(S) * v
+            // (gpuNUFFT_operator.cpp:800-819, std_gpuNUFFT_kernels.cu:
+            // 158-218)
+            float2 v = part_swap<true>(a[j]);
+            v.x = __fmul_rn(v.x, scale);
+            v.y = __fmul_rn(v.y, scale);
+            if (stage_out == 2)
+            {
+              const float d = __ldg(deapo + px);
+              v.x = __fmul_rn(v.x, d);
+              v.y = __fmul_rn(v.y, d);
+            }
+            if (!sum)
+            {
+              out[c * N + (long long)px] = v;
+              continue;
+            }
+            const float2 t = cmul_conj(v, __ldg(sens + c * N + (long long)px));
+            float2 *q = acc + n * kLanes + cl;
+            float2 s = c == c0 ? make_float2(0.f, 0.f) : *q;
+            s.x = __fadd_rn(s.x, t.x);
+            s.y = __fadd_rn(s.y, t.y);
+            if (c + 1 < c1)
+              *q = s;
+            else if (partial)
+              partial[(long long)blockIdx.y * N + (long long)px] = s;
+            else
+            {
+              if (accumulate)
+              {
+                const float2 o = out[px];
+                s = make_float2(o.x + s.x, o.y + s.y);
+              }
+              out[px] = s;
+            }
+          }
+        });
+    __syncthreads();
+  }
+}
+
+// --------------------------------------------------------------------------
+// row passes: lines along x, transposed through shared memory
+// --------------------------------------------------------------------------
+constexpr int kRowPitch = kLanes + 1;
+
+// The block's lines, rows [x][kRowPitch] of `rowbuf` in natural order: the
+// last stage writes them, then whole rows are stored along x.
+__global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
+    k_gen_rows_fwd(const float2 *__restrict__ image,
+                   const float2 *__restrict__ sens,
+                   const float *__restrict__ deapo, Factors f, int Nx,
+                   long long rows, long long N, int C, int in_add,
+                   int out_add, const float2 *__restrict__ roots,
+                   float2 *__restrict__ A)
+{
+  extern __shared__ float2 sm[];
+  float2 *tw = sm, *buf = sm + f.L, *rowbuf = buf + f.L * kRowPitch;
+  fftcore::load_roots(tw, roots, f.L);
+  const long long ln0 = (long long)blockIdx.x * kLanes;  // coil fastest
+  // warps over lines, lanes over x
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5,
+            nw = blockDim.x >> 5;
+  for (int l = warp; l < kLanes; l += nw)
+  {
+    const long long ln = ln0 + l;
+    if (ln >= rows * C)
+      continue;
+    const long long row = (uint32_t)ln / (uint32_t)C;
+    const int c = (int)(ln - row * C);
+    const float2 *ip = image + (sens ? 0 : c * N) + row * Nx;
+    const float2 *mp = sens + c * N + row * Nx;
+    const float *dp = deapo + row * Nx;
+#pragma unroll 4
+    for (int x = lane; x < Nx; x += 32)
+    {
+      float2 v = __ldg(ip + x);
+      if (sens)  // sensMulKernel, then deapodization
+        v = cmul(v, __ldg(mp + x));
+      const float d = __ldg(dp + x);
+      v.x = __fmul_rn(v.x, d);
+      v.y = __fmul_rn(v.y, d);
+      rowbuf[x * kRowPitch + l] = v;
+    }
+  }
+  __syncthreads();
+  const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
+  line_dft<kRowPitch>(
+      f, buf, cl, lt, ln0 + cl < rows * C, tw,
+      [&](int r, int step, auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        r += in_add;
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+          int x = r + j * step;
+          x -= x >= f.L ? f.L : 0;
+          a[j] = x < Nx ? rowbuf[x * kRowPitch + cl] : make_float2(0.f, 0.f);
+        }
+      },
+      [&](int k, int step, auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        k += out_add;
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+          int x = k + j * step;
+          x -= x >= f.L ? f.L : 0;
+          rowbuf[x * kRowPitch + cl] = a[j];
+        }
+      });
+  __syncthreads();
+  for (int l = warp; l < kLanes; l += nw)
+  {
+    const long long ln = ln0 + l;
+    if (ln >= rows * C)
+      continue;
+    const long long row = (uint32_t)ln / (uint32_t)C;
+    const int c = (int)(ln - row * C);
+    float2 *o = A + ((long long)c * rows + row) * f.L;
+#pragma unroll 4
+    for (int x = lane; x < f.L; x += 32)
+      o[x] = rowbuf[x * kRowPitch + l];
+  }
+}
+
+// Block: grid row x 16 coils of one storage group (pitch coils per cell).
+__global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
+    k_gen_xpass(const float2 *__restrict__ grid,
+                const uint32_t *__restrict__ occ, int occ_words, int tile_x,
+                int tile_y, int tile_z, int tiles_y, Geo g, Factors f, int C,
+                int full, int tail, int out_add,
+                const float2 *__restrict__ roots, float2 *__restrict__ out)
+{
+  extern __shared__ float2 sm[];
+  __shared__ uint32_t s_occ[32];
+  float2 *tw = sm, *buf = sm + f.L, *rowbuf = buf + f.L * kRowPitch;
+  const int row = blockIdx.x, grp = blockIdx.y;
+  const int ry = row % g.G[1], rz = row / g.G[1];
+  const int c0 = grp * kLanes;
+  const int pitch = grp < full ? kLanes : tail;
+  const uint32_t *oc =
+      occ +
+      ((size_t)(rz >> tile_z) * tiles_y + (ry >> tile_y)) * occ_words;
+  bool any = false;
+  if (threadIdx.x < 32)
+  {
+    const uint32_t w =
+        (int)threadIdx.x < occ_words ? __ldg(oc + threadIdx.x) : 0u;
+    s_occ[threadIdx.x] = w;
+    any = w != 0u;
+  }
+  fftcore::load_roots(tw, roots, f.L);
+  any = __syncthreads_or(any);
+  int y = ry - g.shift_inv[1], z = rz - g.shift_inv[2];
+  y += y < 0 ? g.G[1] : 0;
+  z += z < 0 ? g.G[2] : 0;
+  const int Nx = g.N[0];
+  const long long plane = (long long)g.G[2] * g.G[1] * Nx;
+  float2 *o = out + (long long)c0 * plane + ((long long)z * g.G[1] + y) * Nx;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5,
+            nw = blockDim.x >> 5;
+  if (!any)
+  {  // no sample reaches this row: its transform is zero
+    for (int l = warp; l < kLanes && c0 + l < C; l += nw)
+      for (int x = lane; x < Nx; x += 32)
+        o[(long long)l * plane + x] = make_float2(0.f, 0.f);
+    return;
+  }
+  const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
+  const float2 *sp =
+      grid + (size_t)c0 * g.grid_count + (size_t)row * f.L * pitch + cl;
+  line_dft<kRowPitch>(
+      f, buf, cl, lt, c0 + cl < C, tw,
+      [&](int r, int step, auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        // FFT input n holds cell (n + floor(G / 2)) mod G
+        r += g.shift_inv[0];
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+          int x = r + j * step;
+          x -= x >= f.L ? f.L : 0;
+          const int t = x >> tile_x;
+          const bool in = (s_occ[t >> 5] >> (t & 31)) & 1u;
+          a[j] = part_swap<true>(in ? __ldg(sp + x * pitch)
+                                    : make_float2(0.f, 0.f));
+        }
+      },
+      [&](int k, int step, auto &a) {
+        constexpr int R = sizeof(a) / sizeof(a[0]);
+        k += out_add;
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+          int x = k + j * step;
+          x -= x >= f.L ? f.L : 0;
+          if (x < Nx)
+            rowbuf[x * kRowPitch + cl] = part_swap<true>(a[j]);
+        }
+      });
+  __syncthreads();
+  for (int l = warp; l < kLanes && c0 + l < C; l += nw)
+#pragma unroll 4
+    for (int x = lane; x < Nx; x += 32)
+      o[(long long)l * plane + x] = rowbuf[x * kRowPitch + l];
+}
+
+template <class K> void set_smem(K k, size_t bytes)
+{
+  if (bytes > 48 * 1024)
+    GN_CUDA(cudaFuncSetAttribute(
+        k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
+Factors factors_of(int L)
+{
+  Factors f;
+  f.L = L;
+  if (!gen_split(L, f.R))
+    throw Error(kInternal, "line length has no transform");
+  // a thread per item of the two-stage lines; the three-stage ones have
+  // more items than a block has threads and loop
+  f.threads = f.R[1] > 1 ? kMaxRadix : std::max(f.R[0], f.R[2]);
+  f.threads += f.threads & 1;  // whole warps
+  return f;
+}
+}  // namespace
+
+bool gen_split(int L, int R[3])
+{
+  // the split into the fewest factors of at most kMaxRadix, the largest
+  // factor as small as possible (fewest idle threads in a stage)
+  int best = 0, a0 = 0, a1 = 0;
+  for (int a = 2; a <= kMaxRadix; ++a)
+    if (L % a == 0 && L / a >= 2 && L / a <= kMaxRadix &&
+        (!best || std::max(a, L / a) < best))
+    {
+      best = std::max(a, L / a);
+      a0 = a;
+    }
+  if (best)
+  {
+    R[0] = std::max(a0, L / a0);
+    R[1] = 1;
+    R[2] = L / R[0];
+    return true;
+  }
+  if (L > 1024)
+    return false;
+  for (int a = 2; a <= kMaxRadix; ++a)
+    for (int b = 2; b <= a; ++b)
+      if (L % (a * b) == 0)
+      {
+        const int c = L / (a * b);
+        if (c >= 2 && c <= b && (!best || a < best))
+        {
+          best = a;
+          a0 = a;
+          a1 = b;
+        }
+      }
+  if (!best)
+    return false;
+  R[0] = a0;
+  R[1] = a1;
+  R[2] = L / (a0 * a1);
+  return true;
+}
+
+void gen_cols(bool inverse, int L, const float2 *src, float2 *dst,
+              long long ncols, int src_rows, int dst_rows, long long planes,
+              int in_add, int in_count, int out_add, int out_count,
+              const float2 *roots, const uint2 *colrange, bool paired,
+              const uint32_t *tiles, int n_tiles, cudaStream_t s)
+{
+  const Factors f = factors_of(L);
+  const int nt = kLanes * f.threads;
+  const int cw = paired ? kLanes / 2 : kLanes;
+  const long long nct = tiles && paired ? n_tiles : (ncols + cw - 1) / cw;
+  const long long ny = paired ? (planes + 1) / 2 : planes;
+  if (nct == 0)
+    return;
+  const size_t smem = (size_t)(L + L * kLanes) * sizeof(float2);
+  auto launch = [&](auto k) {
+    set_smem(k, smem);
+    for (long long p0 = 0; p0 < ny; p0 += 65534)
+    {  // the planes of a launch start on a whole pair
+      const long long n = std::min(ny - p0, 65534LL);
+      const long long first = paired ? 2 * p0 : p0;
+      k<<<dim3((unsigned)nct, (unsigned)n), nt, smem, s>>>(
+          src + first * src_rows * ncols, dst + first * dst_rows * ncols, f,
+          ncols, src_rows, dst_rows, planes - first, in_add, in_count,
+          out_add, out_count, roots, colrange, paired ? tiles : nullptr);
+    }
+  };
+  if (inverse)
+    launch(k_gen_cols<true, false>);
+  else if (paired)
+    launch(k_gen_cols<false, true>);
+  else
+    launch(k_gen_cols<false, false>);
+  GN_LAUNCH_CHECK("general column transform");
+}
+
+void gen_rows_fwd(int L, const float2 *image, const float2 *sens,
+                  const float *deapo, int Nx, long long rows, long long N,
+                  int C, int in_add, int out_add, const float2 *roots,
+                  float2 *A, cudaStream_t s)
+{
+  const Factors f = factors_of(L);
+  const int nt = kLanes * f.threads;
+  const size_t smem = (size_t)(L + 2 * L * kRowPitch) * sizeof(float2);
+  auto k = k_gen_rows_fwd;
+    set_smem(k, smem);
+    k<<<(unsigned)((rows * C + kLanes - 1) / kLanes), nt, smem,
+        s>>>(image, sens, deapo, f, Nx, rows, N, C, in_add, out_add, roots,
+             A);
+  GN_LAUNCH_CHECK("general forward rows");
+}
+
+void gen_cols_sum(int L, const float2 *src, long long ncols,
+                  long long coil_stride, const float *deapo,
+                  const float2 *sens, int n_out, long long N, int C, int cpb,
+                  int groups, int out_add, float scale, int stage,
+                  int accumulate, const float2 *roots, float2 *out,
+                  float2 *partial, cudaStream_t s)
+{
+  const Factors f = factors_of(L);
+  const int nt = kLanes * f.threads;
+  const bool sum = sens != nullptr && stage == 2;
+  const size_t smem =
+      (size_t)(L + (L + (sum ? n_out : 0)) * kLanes) * sizeof(float2);
+  auto k = k_gen_cols_sum;
+    set_smem(k, smem);
+    k<<<dim3((unsigned)((ncols + kLanes - 1) / kLanes), (unsigned)groups),
+        nt, smem, s>>>(src, f, ncols, coil_stride, deapo, sens,
+                                      n_out, N, C, cpb, out_add, scale, stage,
+                                      accumulate, roots, out, partial);
+  GN_LAUNCH_CHECK("general adjoint last pass");
+}
+
+void gen_xpass(const float2 *grid, const uint32_t *occ, int occ_words,
+               int tile_x, int tile_y, int tile_z, int tiles_y, const Geo &g,
+               int C, const float2 *roots, float2 *out, cudaStream_t s)
+{
+  const Factors f = factors_of(g.G[0]);
+  const int L = f.L, nt = kLanes * f.threads;
+  const size_t smem = (size_t)(L + (L + g.N[0]) * kRowPitch) * sizeof(float2);
+  int add = (-(g.crop[0] + g.shift_inv[0])) % L;
+  add += add < 0 ? L : 0;
+  const int full = C / kLanes, rem = C % kLanes;
+  const int tail = rem == 0 ? 0 : (rem <= 4 ? 4 : (rem <= 8 ? 8 : 16));
+  auto k = k_gen_xpass;
+    set_smem(k, smem);
+    k<<<dim3((unsigned)(g.G[1] * g.G[2]), (unsigned)(full + (rem ? 1 : 0))),
+        nt, smem, s>>>(grid, occ, occ_words, tile_x, tile_y,
+                                      tile_z, tiles_y, g, f, C, full, tail,
+                                      add, roots, out);
+  GN_LAUNCH_CHECK("general x transform");
+}
+
+}  // namespace gnufft

@@ -13,6 +13,7 @@
 
 #include "devutil.hpp"
 #include "fftcore.cuh"
+#include "fftgen.cuh"
 #include "tma.cuh"
 
 namespace gnufft
@@ -1141,6 +1142,13 @@ inline int pos_mod(long long v, int m)
   return (int)(r < 0 ? r + m : r);
 }
 
+// Lengths with kernels of their own (with_length); the others take the
+// general passes of fftgen.cu.
+bool pow2_length(int L)
+{
+  return L >= 16 && L <= 1024 && (L & (L - 1)) == 0;
+}
+
 template <class F> void with_length(int L, F &&f)
 {
   switch (L)
@@ -1257,6 +1265,13 @@ void cols(int L, const float2 *src, float2 *dst, long long ncols,
           int list_cols = 0)
 {
   bool done = false;
+  if (!pow2_length(L))
+  {
+    gen_cols(INV, L, src, dst, ncols, src_rows, dst_rows, planes, in_add,
+             in_count, out_add, out_count, roots, colrange, paired,
+             list_cols == kGenTileCols ? tiles : nullptr, (int)n_list, s);
+    return;
+  }
   if (wait.err && L <= 256)
     with_length(L, [&](auto lc) {
       constexpr int LL = decltype(lc)::value;
@@ -1456,14 +1471,20 @@ bool launch_rows_fwd_tma(const float2 *image, const float2 *sens,
 
 }  // namespace
 
-bool pruned_fft_supported(const Geo &g)
+bool pow2_grid(const Geo &g)
 {
   for (int a = 0; a < g.dim; ++a)
-  {
-    const int G = g.G[a];
-    if (G < 16 || G > 1024 || (G & (G - 1)))
+    if (!pow2_length(g.G[a]))
       return false;
-  }
+  return true;
+}
+
+bool pruned_fft_supported(const Geo &g)
+{
+  int R[3];
+  for (int a = 0; a < g.dim; ++a)
+    if (!pow2_length(g.G[a]) && (g.G[a] < 16 || !gen_split(g.G[a], R)))
+      return false;
   return true;
 }
 
@@ -1499,6 +1520,12 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
   const long long N = g.img_count;
   const long long rows = (long long)g.N[1] * g.N[2];
   // x: image rows -> A [C][N_z][N_y][G_x]
+  if (!pow2_length(g.G[0]))
+    gen_rows_fwd(g.G[0], image, sens, deapo, g.N[0], rows, N, C,
+                 pos_mod((long long)g.shift_inv[0] - g.crop[0], g.G[0]),
+                 pos_mod(-(long long)g.shift_fwd[0], g.G[0]), roots[0], tmp_a,
+                 s);
+  else
   with_length(g.G[0], [&](auto lc) {
     constexpr int LL = decltype(lc)::value;
     using S = Shape<LL>;
@@ -1622,21 +1649,33 @@ void launch_pruned_adjoint_xfirst(const float2 *xrows, const float *deapo,
   const long long coil_stride = (long long)g.G[ax] * ncols;
   const int out_add =
       pos_mod(-(long long)g.crop[ax] - g.shift_inv[ax], g.G[ax]);
-  with_length(g.G[ax], [&](auto lc) {
-    constexpr int LL = decltype(lc)::value;
-    using S = Shape<LL>;
-    const long long nb = (ncols + S::TC - 1) / S::TC;
-    // coil groups in separate blocks when the columns alone do not fill
-    // the GPU (eight blocks per SM); their coil sums meet in `partial`
-    int groups = 1;
+  const bool combine = sens != nullptr && stage == 2;
+  // coil groups in separate blocks when the nb blocks of columns alone do
+  // not fill the GPU (eight blocks per SM); their coil sums meet in `partial`
+  int groups = 1, cpb = C;
+  float2 *partial = nullptr;
+  auto split_coils = [&](long long nb) {
     while (groups < C && nb * groups < 148LL * 8)
       groups *= 2;
     if (groups > C)
       groups = C;
-    const int cpb = (C + groups - 1) / groups;
+    cpb = (C + groups - 1) / groups;
     groups = (C + cpb - 1) / cpb;
-    const bool combine = sens != nullptr && stage == 2;
-    float2 *partial = (combine && groups > 1) ? part : nullptr;
+    partial = (combine && groups > 1) ? part : nullptr;
+  };
+  if (!pow2_length(g.G[ax]))
+  {
+    split_coils((ncols + 15) / 16);
+    gen_cols_sum(g.G[ax], src, ncols, coil_stride, deapo, sens, g.N[ax], N, C,
+                 cpb, groups, out_add, g.fft_scale, stage, accumulate,
+                 roots[ax], out, partial, s);
+  }
+  else
+  with_length(g.G[ax], [&](auto lc) {
+    constexpr int LL = decltype(lc)::value;
+    using S = Shape<LL>;
+    const long long nb = (ncols + S::TC - 1) / S::TC;
+    split_coils(nb);
     const dim3 grd((unsigned)nb, (unsigned)groups);
     const bool tiles =
         combine && launch_cols_sum_tma<LL>(src, ncols, coil_stride, deapo,
@@ -1662,13 +1701,13 @@ void launch_pruned_adjoint_xfirst(const float2 *xrows, const float *deapo,
                                          roots[ax], out, nullptr);
     }
     GN_LAUNCH_CHECK("pruned adjoint last pass");
-    if (partial)
-    {
-      k_sum_coil_groups<<<grid_for(N, 256, 148 * 16), 256, 0, s>>>(
-          partial, groups, N, accumulate, out);
-      GN_LAUNCH_CHECK("coil-group sum");
-    }
   });
+  if (partial)
+  {
+    k_sum_coil_groups<<<grid_for(N, 256, 148 * 16), 256, 0, s>>>(
+        partial, groups, N, accumulate, out);
+    GN_LAUNCH_CHECK("coil-group sum");
+  }
 }
 
 size_t pruned_scratch_xfirst(const Geo &g, int C)

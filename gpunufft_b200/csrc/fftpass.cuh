@@ -30,6 +30,10 @@ namespace gnufft
 {
 
 // Every grid axis a power of two in [16, 1024].
+bool pow2_grid(const Geo &g);
+
+// Every grid axis such a power of two or a length of the general passes
+// (fftgen.cuh).  launch_pruned_adjoint needs pow2_grid; the others take all.
 bool pruned_fft_supported(const Geo &g);
 
 // tab[j] = exp(-2 pi i j / L), j < L.

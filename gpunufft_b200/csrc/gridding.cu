@@ -2110,13 +2110,20 @@ using tma::encode_fn;
 
 bool forward_pairs(const Geo &g, int tile_coils)
 {
-  // 3-D, the z transform with tensor-copy tiles (every axis <= 256), kernel
-  // width <= 3 (four footprint slots), tiles of four coils, two pairs of
-  // tiles within three blocks' shared memory per SM
+  // 3-D, the z transform with tensor-copy tiles (power-of-two z <= 256) or
+  // the general one, kernel width <= 3 (four footprint slots), tiles of four
+  // coils, two pairs of tiles within three blocks' shared memory per SM
   if (g.dim != 3 || slots_for(g) != 4 || !encode_fn())
     return false;
+  bool pow2 = true;
   for (int a = 0; a < 3; ++a)
-    if (g.G[a] > 256 || g.G[a] < 16)
+  {
+    if (g.G[a] < 16)
+      return false;
+    pow2 = pow2 && g.pow2G[a];
+  }
+  for (int a = 0; a < 3; ++a)
+    if (g.G[a] > 256 && (pow2 || (a == 2 && g.pow2G[2])))
       return false;
   if (tile_coils > 0 && tile_coils != 4)
     return false;

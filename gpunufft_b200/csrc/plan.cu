@@ -71,6 +71,9 @@ struct gnufft_plan
   bool plain = false;
   int fwd_tile_coils = 0;  // 0: automatic
   bool pruned = false;     // separable pruned transforms instead of cuFFT
+                           // (every grid axis a power of two)
+  bool general = false;    // the general separable passes take the grid
+                           // (calls choose: forward_separable, tile_path)
   // cuFFT grids even along every axis: the forward folds its shift into the
   // prepare pass as signs and reads sector tiles by tensor copies
   bool fwd_signs = false;
@@ -106,7 +109,6 @@ struct gnufft_plan
 
   // per-call scratch (grow-only)
   DeviceBuffer ks, grid, stage_in, stage_out, one_sens, fft_a, fft_b;
-  DeviceBuffer tile_part;  // partial tiles of the tile spread
   std::map<int, cufftHandle> fft;
 
   // timing
@@ -151,7 +153,7 @@ struct gnufft_plan
                                   &stage_out,   &one_sens,    &fft_a,
                                   &fft_b,       &dlut,        &roots[0],
                                   &roots[1],    &roots[2],    &zrange,
-                                  &ztiles,      &tile_part};
+                                  &ztiles};
     size_t s = tiles.bytes();
     for (auto *b : bufs)
       s += b->bytes();
@@ -328,11 +330,13 @@ void init_common(gnufft_plan &p, const gnufft_desc *d)
   if (!gridding_supported(p.g, err))
     throw Error(kNotSupported, err);
   p.pruned = !p.plain && !(d->flags & GNUFFT_FLAG_CUFFT) &&
-             pruned_fft_supported(p.g);
+             pow2_grid(p.g);
+  p.general = !p.plain && !(d->flags & GNUFFT_FLAG_CUFFT) && !p.pruned &&
+              pruned_fft_supported(p.g);
   p.fwd_signs = !p.pruned && !p.plain;
   for (int a = 0; a < p.g.dim; ++a)
     p.fwd_signs = p.fwd_signs && p.g.G[a] % 2 == 0;
-  if (p.pruned || p.fwd_signs)
+  if (p.pruned || p.general || p.fwd_signs)
   {
     GN_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p.copy_err_h),
                           sizeof(int), cudaHostAllocMapped));
@@ -380,6 +384,48 @@ void set_sens_host(gnufft_plan &p, const void *sens, uint32_t n_coils)
   p.sens_coils = n_coils;
 }
 
+// The adjoint of C coils spreads by register columns (tilespread.cuh)
+// instead of the CSR product.  It costs two to four launches more and issues
+// the same instructions per record for 8 coils as for 32; the CSR kernels
+// give a coil count's lanes several entries at once but pay per (sample,
+// cell) pair.  Whole adjoints, CSR -> columns, us on a B200 (M samples,
+// work = CSR entries times coil lanes):
+//   power-of-two grids
+//   3-D, 27 entries a sample: 32^3 image, 16 / 32 coils (work 14 / 28 M)
+//   64 -> 65, 121 -> 102; 64^3, 3 / 8 / 32 coils (28 / 57 / 226 M)
+//   174 -> 133, 237 -> 186, 603 -> 491; 128^3, 32 coils 3899 -> 2928; kernel
+//   width 7 at 64^3 653 -> 339 (4 coils)
+//   2-D, 9 entries: 128^2, 8 / 16 / 32 coils (4 / 7 / 15 M) 33 -> 36,
+//   45 -> 41, 70 -> 52; 256^2, 4 / 8 / 16 / 32 coils (7 / 15 / 30 / 59 M)
+//   46 -> 51, 62 -> 70, 126 -> 104, 211 -> 156; 512^2 (rows of 1024, one CSR
+//   block per SM), 3 / 32 coils 199 -> 159, 1207 -> 605; kernel widths 4 / 5
+//   at 256^2, 3 coils (3 / 4 M) 44 -> 41, 51 -> 43
+//   general grids (the CSR path runs cuFFT and an elementwise pass; the
+//   columns the general passes of fftgen.cuh)
+//   3-D: 72^3 on 108^3, 4 coils (20 M) 192 -> 183; 96^3 on 192^3, 4 / 16 /
+//   32 coils 815 -> 539, 1786 -> 891, 3053 -> 1667; 120^3 on 240^3, 32 coils
+//   7890 -> 3256
+//   2-D kernel width 3: 96^2 on 192^2, 16 / 32 coils (4 / 8 M) 36 -> 42,
+//   53 -> 48; 240^2 on 360^2, 16 / 32 coils (25 / 50 M) 97 -> 112, 196 -> 174;
+//   width 5: 96^2 on 120^2, 8 / 16 coils (6 / 11 M) 37 -> 40, 55 -> 44; 160^2
+//   on 200^2, 4 / 8 coils (8 / 15 M) 42 -> 50, 60 -> 53; 300 x 200, 32 coils
+//   504 -> 246.
+bool tile_rule(const gnufft_plan &p, uint32_t C)
+{
+  if (!(p.pruned || p.general) || !p.copy_err_d || C <= 2 ||
+      !tile_spread_supported(p.g) || !tile_xpass_supported(p.g))
+    return false;
+  const double work = (double)p.nnz * spmm_coil_group((int)C) *
+                      ((C + 31) / 32);
+  if (p.dim == 3)
+    return work >= 20e6;
+  if (p.general)
+    return p.g.kw > 3 ? work >= 11e6 : C > 16 && work >= 6e6;
+  if (p.g.G[0] > 512 || p.g.kw > 3)
+    return work >= 3e6;
+  return C > 8 && work >= 6e6;
+}
+
 void finish_tables(gnufft_plan &p)
 {
   // interpolation matrix (adjoint) and forward work items
@@ -400,10 +446,13 @@ void finish_tables(gnufft_plan &p)
   p.di_inv.reset((size_t)p.M * sizeof(uint32_t) + 4);
   launch_invert_permutation(p.di.as<uint32_t>(), p.M, p.di_inv.as<uint32_t>(),
                             p.stream);
-  if (p.pruned && tile_spread_supported(p.g))
+  // the column spread's records, unless the plan's maps say that its calls
+  // take the CSR product (a plan without maps may be called with any coils)
+  if (p.sens_coils ? tile_rule(p, p.sens_coils)
+                   : (p.pruned || p.general) && tile_spread_supported(p.g))
     build_tile_tables(p.traj_sorted.as<float>(), p.sec_sorted.as<uint32_t>(),
                       p.M, p.g, p.lut.as<float>(), p.tiles, work, p.stream);
-  if (p.pruned && p.dim == 3)
+  if ((p.pruned || p.general) && p.dim == 3)
     build_column_ranges(p.w_rows.as<uint32_t>(), p.g, p.zrange, p.ztiles,
                         p.n_ztiles, p.stream);
   processing_order(p.sdc_h, p.order_h);
@@ -609,39 +658,30 @@ std::array<const float2 *, 3> root_ptrs(const gnufft_plan &p)
           p.roots[2].as<float2>()};
 }
 
-// The adjoint of C coils spreads by register columns (tilespread.cuh)
-// instead of the CSR product.  It costs two to four launches more and issues
-// the same instructions per record for 8 coils as for 32; the CSR kernels
-// give a coil count's lanes several entries at once but pay per (sample,
-// cell) pair.  Whole adjoints, CSR -> columns, us on a B200 (M samples,
-// entries x lanes = CSR entries times coil lanes):
-//   3-D, 27 entries a sample: 32^3 image, 16 / 32 coils (14 / 28 M entries x
-//   lanes) 64 -> 65, 121 -> 102; 64^3, 3 / 8 / 32 coils (28 / 57 / 226 M)
-//   174 -> 133, 237 -> 186, 603 -> 491; 128^3, 32 coils 3899 -> 2928; kernel
-//   width 7 at 64^3 653 -> 339 (4 coils)
-//   2-D, 9 entries: 128^2, 8 / 16 / 32 coils (4 / 7 / 15 M) 33 -> 36,
-//   45 -> 41, 70 -> 52; 256^2, 4 / 8 / 16 / 32 coils (7 / 15 / 30 / 59 M)
-//   46 -> 51, 62 -> 70, 126 -> 104, 211 -> 156; 512^2 (rows of 1024, one CSR
-//   block per SM), 3 / 32 coils 199 -> 159, 1207 -> 605; kernel widths 4 / 5
-//   at 256^2, 3 coils (3 / 4 M) 44 -> 41, 51 -> 43.
 bool tile_path(const gnufft_plan &p, uint32_t C)
 {
-  if (!p.pruned || !p.copy_err_d || !p.tiles.ready() || C <= 2 ||
-      !tile_xpass_supported(p.g))
-    return false;
-  const double work = (double)p.nnz * spmm_coil_group((int)C) *
-                      ((C + 31) / 32);
-  if (p.dim == 3)
-    return work >= 20e6;
-  if (p.g.G[0] > 512 || p.g.kw > 3)
-    return work >= 3e6;
-  return C > 8 && work >= 6e6;
+  return p.tiles.ready() && tile_rule(p, C);
+}
+
+// The forward of C coils runs separable passes.  On general grids cuFFT's
+// passes over the zero-padded grid are kept where the image is small next to
+// the launches or the coil-pair grid would be half empty (whole forwards,
+// cuFFT -> separable, us on a B200): 96^3 on 192^3, 1 / 4 / 16 / 32 coils
+// 137 -> 205, 500 -> 362, 1850 -> 975, 3657 -> 1820; 88 x 88 x 44 on 132 x
+// 132 x 66, 4 coils 128 -> 124; 120^3 on 240^3, 32 coils 8756 -> 3494; with
+// an odd axis (no tensor-copy tiles either way) 100^3 on 125^3, 4 / 32 coils
+// 449 -> 463, 4777 -> 4753; 2-D 240^2 on 360^2, 4 / 16 / 32 coils 30 -> 38,
+// 69 -> 69, 133 -> 146.
+bool forward_separable(const gnufft_plan &p, uint32_t C)
+{
+  return p.pruned || (p.general && p.dim == 3 && C >= 4 && p.fwd_signs);
 }
 
 // The forward's grid holds coil pairs interleaved (3-D separable path).
-bool paired_grid(const gnufft_plan &p)
+bool paired_grid(const gnufft_plan &p, uint32_t C)
 {
-  return p.pruned && p.copy_err_d && forward_pairs(p.g, p.fwd_tile_coils);
+  return forward_separable(p, C) && p.copy_err_d &&
+         forward_pairs(p.g, p.fwd_tile_coils);
 }
 
 // Complex elements of the adjoint's x-transformed rows.
@@ -684,10 +724,11 @@ void adjoint_batched(gnufft_plan &p, const float2 *k, float2 *img, uint32_t C,
     check_copy_err(p);
     ensure_pruned(p, C, s);
     p.fft_b.ensure(xrows_elems(g, C) * sizeof(float2));
-    p.tile_part.ensure(tile_partial_elems(p.tiles, g, (int)C) * sizeof(float2));
+    // the partial columns live in the buffer of the coil-group sums, which
+    // come later
+    p.fft_a.ensure(tile_partial_elems(p.tiles, g, (int)C) * sizeof(float2));
     p.launches += launch_tile_spread(p.tiles, p.ks.as<float2>(), CP, g,
-                                     (int)C, grid, p.tile_part.as<float2>(),
-                                     s);
+                                     (int)C, grid, p.fft_a.as<float2>(), s);
     p.mark(3, s);
     p.mark(4, s);
     launch_tile_xpass(p.tiles, grid, g, (int)C, p.roots[0].as<float2>(),
@@ -783,11 +824,12 @@ void forward_batched(gnufft_plan &p, const float2 *img, float2 *k, uint32_t C,
   }
   const bool dens_est = stage == GNUFFT_DENSITY_ESTIMATION;
   // 3-D pruned path: the grid holds coil pairs interleaved
-  const bool paired = !dens_est && paired_grid(p);
+  const bool separable = !dens_est && forward_separable(p, C);
+  const bool paired = !dens_est && paired_grid(p, C);
   p.grid.ensure((size_t)(paired ? (C + 1) / 2 * 2 : C) * g.grid_count *
                 sizeof(float2));
   float2 *grid = p.grid.as<float2>();
-  if (p.pruned && !dens_est)
+  if (separable)
   {  // sens, deapodization, pad, shift and the transform in g.dim passes
     check_copy_err(p);
     ensure_pruned(p, C, s);
@@ -892,27 +934,29 @@ void traj_grad(gnufft_plan &p, const float2 *img, const float2 *u, uint32_t C,
 // Complex elements that one call with C coils needs of each scratch buffer.
 struct ScratchNeeds
 {
-  size_t ks = 0, grid = 0, fft_a = 0, fft_b = 0, tile_part = 0;
+  size_t ks = 0, grid = 0, fft_a = 0, fft_b = 0;
+  bool cufft = false;  // the call runs cuFFT (its plan holds a work area)
   void merge(const ScratchNeeds &o)
   {
     ks = std::max(ks, o.ks);
     grid = std::max(grid, o.grid);
     fft_a = std::max(fft_a, o.fft_a);
     fft_b = std::max(fft_b, o.fft_b);
-    tile_part = std::max(tile_part, o.tile_part);
+    cufft = cufft || o.cufft;
   }
   size_t bytes() const
   {
-    return (ks + grid + fft_a + fft_b + tile_part) * sizeof(float2);
+    return (ks + grid + fft_a + fft_b) * sizeof(float2);
   }
 };
 
 ScratchNeeds forward_needs(const gnufft_plan &p, uint32_t C)
 {
   ScratchNeeds n;
-  n.grid = (size_t)(paired_grid(p) ? (C + 1) / 2 * 2 : C) *
+  n.grid = (size_t)(paired_grid(p, C) ? (C + 1) / 2 * 2 : C) *
            (size_t)p.g.grid_count;
-  if (p.pruned)
+  n.cufft = !forward_separable(p, C);
+  if (!n.cufft)
   {
     n.fft_a = pruned_scratch_a(p.g, (int)C);
     n.fft_b = std::max(pruned_scratch_b(p.g, (int)C),
@@ -928,9 +972,10 @@ ScratchNeeds adjoint_needs(const gnufft_plan &p, uint32_t C)
   ScratchNeeds n;
   n.ks = (size_t)p.M * ((C + cg - 1) / cg * cg);
   const bool tiled = tile_path(p, C);
+  n.cufft = !tiled && !p.pruned;
   n.grid = (size_t)(tiled ? tile_grid_pitch((int)C) : (int)C) *
            (size_t)g.grid_count;
-  if (p.pruned)
+  if (!n.cufft)
   {
     n.fft_a = pruned_scratch_a(g, (int)C);
     n.fft_b = std::max(pruned_scratch_b(g, (int)C),
@@ -939,7 +984,7 @@ ScratchNeeds adjoint_needs(const gnufft_plan &p, uint32_t C)
   if (tiled)
   {
     n.fft_b = std::max(n.fft_b, xrows_elems(g, C));
-    n.tile_part = tile_partial_elems(p.tiles, g, (int)C);
+    n.fft_a = std::max(n.fft_a, tile_partial_elems(p.tiles, g, (int)C));
   }
   return n;
 }
@@ -951,7 +996,7 @@ size_t call_scratch_bytes(const gnufft_plan &p, uint32_t C)
   ScratchNeeds n = forward_needs(p, C);
   n.merge(adjoint_needs(p, C));
   size_t b = n.bytes();
-  if (!p.pruned)
+  if (n.cufft)
     b += (size_t)C * p.g.grid_count * sizeof(float2);
   return b;
 }
@@ -964,14 +1009,13 @@ bool scratch_held(const gnufft_plan &p, const ScratchNeeds &n, uint32_t C)
     return b.bytes() >= elems * sizeof(float2);
   };
   return has(p.ks, n.ks) && has(p.grid, n.grid) && has(p.fft_a, n.fft_a) &&
-         has(p.fft_b, n.fft_b) && has(p.tile_part, n.tile_part) &&
-         (p.pruned || p.fft.count((int)C) != 0);
+         has(p.fft_b, n.fft_b) &&
+         (!n.cufft || p.fft.count((int)C) != 0);
 }
 
 size_t held_scratch_bytes(const gnufft_plan &p)
 {
-  return p.ks.bytes() + p.grid.bytes() + p.fft_a.bytes() + p.fft_b.bytes() +
-         p.tile_part.bytes();
+  return p.ks.bytes() + p.grid.bytes() + p.fft_a.bytes() + p.fft_b.bytes();
 }
 
 // Coils per pass so that a pass's scratch fits the plan's memory limit, or

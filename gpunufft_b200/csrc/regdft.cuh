@@ -1,0 +1,207 @@
+// In-register DFTs of any length up to 32 (forward sign, natural order in
+// and out): Cooley-Tukey splits down to primes, every twiddle a compile-time
+// constant; a prime length P takes the sums and differences of the pairs
+// (j, P - j) and (P - 1)^2 / 2 real multiply-adds per part.
+#pragma once
+
+#include <utility>
+
+#include <cuda_runtime.h>
+
+namespace gnufft
+{
+namespace regdft
+{
+// cos(2 pi m / n), sin(2 pi m / n) in double by octant reduction and the
+// Taylor series (arguments up to pi / 4, terms to 1e-19).
+constexpr double kPi = 3.14159265358979323846264338327950288;
+
+__host__ __device__ constexpr double taylor_sin(double x)
+{
+  double t = x, s = x;
+  for (int i = 1; i < 12; ++i)
+  {
+    t *= -x * x / ((2.0 * i) * (2.0 * i + 1.0));
+    s += t;
+  }
+  return s;
+}
+
+__host__ __device__ constexpr double taylor_cos(double x)
+{
+  double t = 1.0, s = 1.0;
+  for (int i = 1; i < 12; ++i)
+  {
+    t *= -x * x / ((2.0 * i - 1.0) * (2.0 * i));
+    s += t;
+  }
+  return s;
+}
+
+struct CosSin
+{
+  double c, s;
+};
+
+__host__ __device__ constexpr CosSin cos_sin(int m, int n)
+{
+  m %= n;
+  if (m < 0)
+    m += n;
+  // octant: angle = 2 pi m / n = (pi / 4) o + rest
+  const int o = (8 * m) / n;
+  const double rest = 2.0 * kPi * (double)(8 * m - o * n) / (8.0 * n);
+  const double up = kPi / 4 - rest;  // used in odd octants
+  const double c = o & 1 ? taylor_sin(up) : taylor_cos(rest);
+  const double s = o & 1 ? taylor_cos(up) : taylor_sin(rest);
+  switch (o)
+  {
+  case 0: return CosSin{c, s};
+  case 1: return CosSin{c, s};
+  case 2: return CosSin{-s, c};
+  case 3: return CosSin{-s, c};
+  case 4: return CosSin{-c, -s};
+  case 5: return CosSin{-c, -s};
+  case 6: return CosSin{s, -c};
+  default: return CosSin{s, -c};
+  }
+}
+
+template <int... I, class F>
+__device__ __forceinline__ void for_seq(std::integer_sequence<int, I...>, F f)
+{
+  (f(std::integral_constant<int, I>()), ...);
+}
+// f(integral_constant 0), ..., f(integral_constant N - 1)
+template <int N, class F> __device__ __forceinline__ void static_for(F f)
+{
+  for_seq(std::make_integer_sequence<int, N>(), f);
+}
+
+// v * exp(-2 pi i M / N)
+template <int M, int N> __device__ __forceinline__ float2 twiddle(float2 v)
+{
+  constexpr int m = M % N;
+  if constexpr (m == 0)
+    return v;
+  else if constexpr (2 * m == N)
+    return make_float2(-v.x, -v.y);
+  else if constexpr (4 * m == N)
+    return make_float2(v.y, -v.x);
+  else if constexpr (4 * m == 3 * N)
+    return make_float2(-v.y, v.x);
+  else
+  {
+    constexpr CosSin w = cos_sin(m, N);
+    constexpr float c = (float)w.c, s = (float)w.s;
+    return make_float2(__fmaf_rn(v.x, c, __fmul_rn(v.y, s)),
+                       __fmaf_rn(v.y, c, -__fmul_rn(v.x, s)));
+  }
+}
+
+// The first factor A of the split R = A * B: 4 where it divides, else the
+// smallest prime factor; 1 for a prime.
+__host__ __device__ constexpr int split_of(int R)
+{
+  if (R % 4 == 0 && R > 4)
+    return 4;
+  for (int p = 2; p * p <= R; ++p)
+    if (R % p == 0)
+      return p;
+  return 1;  // prime
+}
+
+template <int R> struct Dft
+{
+  __device__ static __forceinline__ void run(float2 (&a)[R])
+  {
+    constexpr int A = split_of(R);
+    if constexpr (R == 1)
+    {
+    }
+    else if constexpr (R == 2)
+    {
+      const float2 u = a[0], v = a[1];
+      a[0] = make_float2(u.x + v.x, u.y + v.y);
+      a[1] = make_float2(u.x - v.x, u.y - v.y);
+    }
+    else if constexpr (A == 1)
+    {  // odd prime
+      constexpr int H = (R - 1) / 2;
+      float2 t[H], d[H];
+      float2 sum = a[0];
+      static_for<H>([&](auto jc) {
+        constexpr int j = decltype(jc)::value + 1;
+        const float2 u = a[j], v = a[R - j];
+        t[j - 1] = make_float2(u.x + v.x, u.y + v.y);
+        d[j - 1] = make_float2(u.x - v.x, u.y - v.y);
+        sum = make_float2(sum.x + t[j - 1].x, sum.y + t[j - 1].y);
+      });
+      const float2 a0 = a[0];
+      a[0] = sum;
+      static_for<H>([&](auto kc) {
+        constexpr int k = decltype(kc)::value + 1;
+        float2 re = a0, im = make_float2(0.f, 0.f);
+        static_for<H>([&](auto jc) {
+          constexpr int j = decltype(jc)::value + 1;
+          constexpr CosSin w = cos_sin(j * k, R);
+          constexpr float c = (float)w.c, s = (float)w.s;
+          re = make_float2(__fmaf_rn(t[j - 1].x, c, re.x),
+                           __fmaf_rn(t[j - 1].y, c, re.y));
+          im = make_float2(__fmaf_rn(d[j - 1].x, s, im.x),
+                           __fmaf_rn(d[j - 1].y, s, im.y));
+        });
+        // X_k = re - i im, X_{R-k} = re + i im
+        a[k] = make_float2(re.x + im.y, re.y - im.x);
+        a[R - k] = make_float2(re.x - im.y, re.y + im.x);
+      });
+    }
+    else
+    {
+      // n = B n1 + n2 (n1 < A, n2 < B), X[k1 + A k2]
+      constexpr int B = R / A;
+      float2 b[R];
+      static_for<B>([&](auto n2c) {
+        constexpr int n2 = decltype(n2c)::value;
+        float2 c[A];
+        static_for<A>([&](auto n1c) {
+          constexpr int n1 = decltype(n1c)::value;
+          c[n1] = a[B * n1 + n2];
+        });
+        if constexpr (A == 4)
+        {
+          const float2 s0 = make_float2(c[0].x + c[2].x, c[0].y + c[2].y);
+          const float2 s1 = make_float2(c[0].x - c[2].x, c[0].y - c[2].y);
+          const float2 s2 = make_float2(c[1].x + c[3].x, c[1].y + c[3].y);
+          const float2 s3 = make_float2(c[1].x - c[3].x, c[1].y - c[3].y);
+          c[0] = make_float2(s0.x + s2.x, s0.y + s2.y);
+          c[2] = make_float2(s0.x - s2.x, s0.y - s2.y);
+          c[1] = make_float2(s1.x + s3.y, s1.y - s3.x);
+          c[3] = make_float2(s1.x - s3.y, s1.y + s3.x);
+        }
+        else
+          Dft<A>::run(c);
+        static_for<A>([&](auto k1c) {
+          constexpr int k1 = decltype(k1c)::value;
+          b[k1 * B + n2] = twiddle<n2 * k1, R>(c[k1]);
+        });
+      });
+      static_for<A>([&](auto k1c) {
+        constexpr int k1 = decltype(k1c)::value;
+        float2 c[B];
+        static_for<B>([&](auto n2c) {
+          constexpr int n2 = decltype(n2c)::value;
+          c[n2] = b[k1 * B + n2];
+        });
+        Dft<B>::run(c);
+        static_for<B>([&](auto k2c) {
+          constexpr int k2 = decltype(k2c)::value;
+          a[k1 + A * k2] = c[k2];
+        });
+      });
+    }
+  }
+};
+
+}  // namespace regdft
+}  // namespace gnufft

@@ -20,6 +20,7 @@
 #include "binning.cuh"
 #include "f32x2.cuh"
 #include "fftcore.cuh"
+#include "fftgen.cuh"
 #include "footprint.cuh"
 
 namespace gnufft
@@ -1117,7 +1118,8 @@ int launch_tile_spread(const TileTables &t, const float2 *ks, int CP,
 bool tile_xpass_supported(const Geo &g)
 {
   const int L = g.G[0];
-  return L >= 16 && L <= 1024 && (L & (L - 1)) == 0;
+  int R[3];
+  return (L >= 16 && L <= 1024 && (L & (L - 1)) == 0) || gen_split(L, R);
 }
 
 void launch_tile_xpass(const TileTables &t, const float2 *grid,
@@ -1128,6 +1130,13 @@ void launch_tile_xpass(const TileTables &t, const float2 *grid,
   const int ty = fftcore::ilog2(g.dim == 3 ? Tile<3>::Y : Tile<2>::Y);
   const int tz = fftcore::ilog2(g.dim == 3 ? Tile<3>::Z : Tile<2>::Z);
   const int tiles_y = (g.G[1] + (1 << ty) - 1) >> ty;
+  if (g.G[0] & (g.G[0] - 1))
+  {
+    gen_xpass(grid, t.occ.as<uint32_t>(), occ_words_of(g),
+              fftcore::ilog2(tile_x(g)), ty, tz, tiles_y, g, C, roots_x, out,
+              s);
+    return;
+  }
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

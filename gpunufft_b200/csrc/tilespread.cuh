@@ -78,7 +78,7 @@ int launch_tile_spread(const TileTables &t, const float2 *ks, int CP,
 
 // The inverse x transform of the spread's grid: out [C][G_z][G_y][N_x]
 // (rows in the INVERSE-shifted frame the next passes expect), for
-// power-of-two rows of 16 to 1024 cells.
+// power-of-two rows of 16 to 1024 cells and those of the general passes.
 bool tile_xpass_supported(const Geo &g);
 void launch_tile_xpass(const TileTables &t, const float2 *grid,
                        const Geo &g, int C, const float2 *roots_x,

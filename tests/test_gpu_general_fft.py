@@ -1,0 +1,136 @@
+"""The general separable passes (line lengths that are no power of two)
+against cuFFT, coil by coil (plain plans)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+import gpunufft_b200 as G  # noqa: E402
+from oracle import nufft_oracle as O  # noqa: E402
+
+
+def _rel(a, b):
+    return float(torch.linalg.vector_norm(a - b) /
+                 torch.linalg.vector_norm(b))
+
+
+# image, osf, kernel width, coils, maps.  Grid axes (x, y, z) in the comments:
+# two factors (24 = 6 x 4, 36, 52 = 13 x 4, 66 = 11 x 6, 110, 150 = 15 x 10,
+# 240 = 16 x 15), three (264, 352, 400, 450), odd lengths (25, 27, 39, 45,
+# 75), powers of two beside them; partial blocks of columns, coil counts with
+# and without a partial 16-coil group
+FORWARD = [
+    ((12, 18, 26), 2.0, 3, 4, True),     # 24 x 36 x 52
+    ((66, 32, 20), 1.0, 3, 5, False),    # 66 x 32 x 20
+    ((176, 16, 12), 1.5, 3, 17, True),   # 264 x 24 x 18
+    ((16, 100, 20), 1.5, 3, 7, True),    # 24 x 150 x 30
+    ((24, 24, 200), 2.0, 3, 6, False),   # 48 x 48 x 400
+    ((24, 176, 16), 2.0, 3, 9, True),    # 48 x 352 x 32
+    ((20, 40, 30), 1.2, 5, 8, True),     # 24 x 48 x 36, 8 footprint slots
+]
+
+
+@pytest.mark.parametrize("dims,osf,kw,C,maps", FORWARD)
+def test_general_forward(dims, osf, kw, C, maps):
+    rng = np.random.default_rng(3)
+    shape = dims[::-1]
+    M = 6000
+    traj = rng.uniform(-0.5, 0.4999, (3, M)).astype(np.float32)
+    traj[:, :1500] *= 0.1
+    sens = None
+    if maps:
+        sens = (rng.standard_normal((C,) + shape) + 1j * rng.standard_normal(
+            (C,) + shape)).astype(np.complex64)
+    n = 1 if maps else C
+    x = (rng.standard_normal((n,) + shape) + 1j * rng.standard_normal(
+        (n,) + shape)).astype(np.complex64)
+    xt = torch.from_numpy(x).cuda()
+    p = G.Plan(traj, dims, kw, 8, osf, None, sens)
+    ref = G.Plan(traj, dims, kw, 8, osf, None, sens, plain=True)
+    got = p.forward(xt if not maps else xt[0], n_coils=C)
+    assert p.stage_times()["launches"] == 4  # x, y, z, interpolation
+    want = ref.forward(xt if not maps else xt[0], n_coils=C)
+    # both paths against the float64 oracle.  Rounding is 6e-8 per butterfly
+    # step, some 30 steps, in quadrature; without oversampling (osf 1) the
+    # deapodization's large edge values cancel in the interpolation, which
+    # amplifies it alike on both paths: the cuFFT path's own distance from
+    # the oracle is the bound there
+    exact = torch.from_numpy(O.OracleOperator(
+        traj, dims, kw, 8, osf, sens=sens).forward(x)).cuda()
+    err, err_ref = _rel(got, exact), _rel(want, exact)
+    assert err < max(1e-6, 1.5 * err_ref), (err, err_ref)
+    p.close()
+    ref.close()
+
+
+ADJOINT = [
+    ((12, 18, 26), 2.0, 3, 32, 30000, True),     # 24 x 36 x 52
+    ((25, 39, 45), 1.0, 3, 11, 60000, False),    # 25 x 39 x 45
+    ((176, 16, 16), 1.5, 3, 17, 26000, True),    # 264 x 24 x 24
+    ((16, 100, 20), 1.5, 5, 6, 30000, True),     # 24 x 150 x 30
+    ((24, 24, 200), 2.0, 3, 40, 14000, False),   # 48 x 48 x 400
+    ((44, 300, 16), 1.5, 3, 20, 30000, True),    # 66 x 450 x 24
+    ((33, 32, 160), 2.0, 3, 4, 200000, False),   # 66 x 64 x 320
+    ((160, 220), 1.5, 3, 20, 40000, True),       # 240 x 330
+    ((60, 32), 1.25, 5, 8, 70000, False),        # 75 x 40
+    ((110, 135), 2.0, 5, 33, 16000, True),       # 220 x 270
+]
+
+
+@pytest.mark.parametrize("dims,osf,kw,C,M,maps", ADJOINT)
+def test_general_adjoint(dims, osf, kw, C, M, maps):
+    rng = np.random.default_rng(4)
+    shape = dims[::-1]
+    traj = rng.uniform(-0.5, 0.4999, (len(dims), M)).astype(np.float32)
+    traj[:, :M // 4] *= 0.1
+    dens = rng.uniform(0.1, 1.0, M).astype(np.float32)
+    sens = None
+    if maps:
+        sens = (rng.standard_normal((C,) + shape) + 1j * rng.standard_normal(
+            (C,) + shape)).astype(np.complex64)
+    k = (rng.standard_normal((C, M)) + 1j * rng.standard_normal(
+        (C, M))).astype(np.complex64)
+    kt = torch.from_numpy(k).cuda()
+    p = G.Plan(traj, dims, kw, 8, osf, dens, sens)
+    ref = G.Plan(traj, dims, kw, 8, osf, dens, sens, plain=True)
+    got = p.adjoint(kt)
+    # gather, column spread, the axes' passes (and reductions); the path over
+    # cuFFT has three launches of the library's own
+    assert p.stage_times()["launches"] >= 2 + len(dims)
+    assert torch.equal(got, p.adjoint(kt))
+    # rounding as above; without maps the image is the FFT stage times the
+    # deapodization d, so an error e of that stage becomes at most max(d) e
+    # (osf 1: max(d) is 1000 and the large pixels are the small ones of the
+    # stage); with maps and osf > 1 d varies by less than ten
+    fft, want_fft = p.adjoint(kt, G.FFT), ref.adjoint(kt, G.FFT)
+    assert _rel(fft, want_fft) < 2e-6
+    want = ref.adjoint(kt)
+    tol = 2e-6
+    if osf == 1.0:
+        tol *= float(p.tables()["deapo"].max() *
+                     torch.linalg.vector_norm(want_fft) /
+                     torch.linalg.vector_norm(want))
+    assert _rel(got, want) < tol
+    p.close()
+    ref.close()
+
+
+def test_few_coils_and_memory_limit_on_a_general_grid():
+    """Coil counts on both sides of the separable forward's limit, and a
+    memory limit that splits the call, give the same values."""
+    rng = np.random.default_rng(5)
+    dims, M, C = (24, 20, 36), 30000, 12
+    traj = rng.uniform(-0.5, 0.4999, (3, M)).astype(np.float32)
+    x = torch.from_numpy((rng.standard_normal((C, 36, 20, 24)) +
+                          1j * rng.standard_normal((C, 36, 20, 24))).astype(
+                              np.complex64)).cuda()
+    p = G.Plan(traj, dims)
+    y = p.forward(x)
+    assert _rel(p.forward(x[:3]), y[:3]) < 2e-6
+    a = p.adjoint(y)
+    assert _rel(p.adjoint(y[:2].contiguous()), a[:2]) < 2e-6
+    p.set_memory_limit(p.call_scratch_bytes(5))
+    assert _rel(p.forward(x), y) < 2e-6
+    assert _rel(p.adjoint(y), a) < 2e-6
+    p.close()
