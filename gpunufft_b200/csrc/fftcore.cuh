@@ -91,24 +91,44 @@ __host__ __device__ constexpr int ilog2(int v)
 // w[k] = exp(-2 pi i k / RM), k < RM / 2, RM >= R (conjugated for the
 // inverse).  Every loop has a constant trip count and every index is a
 // constant, so data and roots stay in registers.
-template <int R, int RM, bool INV>
+// MID_ZERO: inputs R / 4 .. 3 R / 4 - 1 are zero (and not read), so that the
+// first butterflies, which pair inputs R / 2 apart, are copies.
+template <int R, int RM, bool INV, bool MID_ZERO = false>
 __device__ __forceinline__ void reg_fft(float2 (&a)[R],
                                         const float2 (&w)[RM / 2])
 {
-#pragma unroll
-  for (int i = 0; i < R; ++i)
+  if constexpr (MID_ZERO)
   {
-    const int j = bitrev(i, R);
-    if (j > i)
+    float2 t[R];
+#pragma unroll
+    for (int b = 0; b < R / 2; ++b)
     {
-      const float2 t = a[i];
-      a[i] = a[j];
-      a[j] = t;
+      const int j = bitrev(2 * b, R);  // < R / 2; its partner is j + R / 2
+      const float2 u = j < R / 4 ? a[j] : a[j + R / 2];
+      t[2 * b] = u;
+      t[2 * b + 1] = j < R / 4 ? u : make_float2(-u.x, -u.y);
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      a[i] = t[i];
+  }
+  else
+  {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+    {
+      const int j = bitrev(i, R);
+      if (j > i)
+      {
+        const float2 t = a[i];
+        a[i] = a[j];
+        a[j] = t;
+      }
     }
   }
   constexpr int LOG = ilog2(R);
 #pragma unroll
-  for (int st = 0; st < LOG; ++st)
+  for (int st = MID_ZERO ? 1 : 0; st < LOG; ++st)
   {
     const int half = 1 << st;
 #pragma unroll
@@ -150,21 +170,21 @@ template <int L> struct Rm
   static constexpr int V = Shape<L>::T;  // roots kept for the larger DFT
 };
 
-template <int L, bool INV, int YS>
+template <int L, bool INV, int YS, bool MID_ZERO = false>
 __device__ __forceinline__ void stage1(float2 (&a)[Shape<L>::R1], int lt,
                                        const float2 (&w)[Rm<L>::V / 2],
                                        const float2 *__restrict__ tw,
                                        float2 *__restrict__ Y)
 {
   using S = Shape<L>;
-  reg_fft<S::R1, Rm<L>::V, INV>(a, w);
+  reg_fft<S::R1, Rm<L>::V, INV, MID_ZERO>(a, w);
 #pragma unroll
   for (int k1 = 0; k1 < S::R1; ++k1)
   {
     float2 v = a[k1];
     if (k1 != 0)
     {
-      float2 r = tw[(lt * k1) & (L - 1)];
+      float2 r = tw[lt * k1];  // lt < R2, k1 < R1: below L
       if (INV)
         r.y = -r.y;
       v = cmul(v, r);
@@ -184,6 +204,28 @@ __device__ __forceinline__ void stage2(float2 (&b)[Shape<L>::R2], int lt,
   for (int t = 0; t < S::R2; ++t)
     b[t] = Y[(lt * S::YP + t) * YS];
   reg_fft<S::R2, Rm<L>::V, INV>(b, w);
+}
+
+// Axes oversampled by two (N = L / 2, crop L / 4: HALF kernels).  Forward:
+// FFT inputs n < L / 4 and n >= 3 L / 4 hold the image, the others are zero;
+// inverse: these outputs are the image.  With n = lt + S j (S the stage
+// stride, R values a thread) these are the j < R / 4 and j >= 3 R / 4, and
+// image row n + L / 4 (mod L) is lt + S times a constant.  Half the loads or
+// stores, their range tests and the first or last butterflies go away (us on
+// a B200): 2-D 256^2 x 16, 512-point lines, rows 37.7 -> 13.9, columns 20.8 ->
+// 17.1, last adjoint pass 21.1 -> 19.3; 3-D 64^3 x 8, y 24.3 -> 20.3, z 37.1 ->
+// 33.6, adjoint y 23.0 -> 20.3, last 18.3 -> 15.9; 3-D 128^3 x 32, z 814 ->
+// 778, last adjoint pass 310 -> 277; the plain 256-point column passes, which
+// move their bytes at the DRAM rate, 603 -> 640 and 540 -> 594: those keep the
+// general form.
+__host__ __device__ constexpr bool half_in(int j, int R)
+{
+  return j < R / 4 || j >= 3 * R / 4;
+}
+// image row of value j: lt + S * half_row(j, R)
+__host__ __device__ constexpr int half_row(int j, int R)
+{
+  return j < R / 4 ? j + R / 4 : j - 3 * R / 4;
 }
 
 template <int L>

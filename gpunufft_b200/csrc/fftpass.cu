@@ -28,7 +28,7 @@ using namespace fftcore;
 // src: planes of src_rows x ncols, dst: planes of dst_rows x ncols.  FFT
 // input n reads source row (n + in_add) mod L when < in_count (else zero);
 // FFT output k goes to row (k + out_add) mod L when < out_count.
-template <int L, bool INV>
+template <int L, bool INV, bool HALF>
 __global__ void __launch_bounds__(Shape<L>::CT)
     k_fft_cols(const float2 *__restrict__ src, float2 *__restrict__ dst,
                long long ncols, int src_rows, int dst_rows, int in_add,
@@ -62,11 +62,19 @@ __global__ void __launch_bounds__(Shape<L>::CT)
 #pragma unroll
     for (int j = 0; j < S::R1; ++j)
     {
+      if (HALF && !INV)
+      {
+        if (half_in(j, S::R1))
+          a[j] = on ? __ldg(sp + (long long)(lt + S::R2 * half_row(j, S::R1)) *
+                                     ncols)
+                    : make_float2(0.f, 0.f);
+        continue;
+      }
       const int r = (lt + S::R2 * j + in_add) & (L - 1);
       a[j] = (on && r < in_count) ? __ldg(sp + (long long)r * ncols)
                                   : make_float2(0.f, 0.f);
     }
-    stage1<L, INV, S::TC>(a, lt, w, tw, Y);
+    stage1<L, INV, S::TC, HALF && !INV>(a, lt, w, tw, Y);
   }
   __syncthreads();
   if (lt < S::R1)
@@ -78,6 +86,12 @@ __global__ void __launch_bounds__(Shape<L>::CT)
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
       {
+        if (HALF && INV)
+        {
+          if (half_in(k2, S::R2))
+            dp[(long long)(lt + S::R1 * half_row(k2, S::R2)) * ncols] = b[k2];
+          continue;
+        }
         const int r = (lt + S::R1 * k2 + out_add) & (L - 1);
         if (r < out_count && (unsigned)r >= cr.x && (unsigned)r <= cr.y)
           dp[(long long)r * ncols] = b[k2];
@@ -139,7 +153,8 @@ __device__ __forceinline__ int col_pos(int r, int cl)
     return r * TC + cl;
 }
 
-template <int L, bool INV, bool PAIRS = false>
+// HALF: see fftcore::half_in (forward: the tile holds the N image rows).
+template <int L, bool INV, bool PAIRS = false, bool HALF = false>
 __device__ __forceinline__ void col_tile_fft(float2 *B, int cl, int lt,
                                              int in_add, int in_count,
                                              const float2 (&w)[Rm<L>::V / 2],
@@ -153,18 +168,25 @@ __device__ __forceinline__ void col_tile_fft(float2 *B, int cl, int lt,
 #pragma unroll
     for (int j = 0; j < S::R1; ++j)
     {
+      if (HALF && !INV)
+      {
+        if (half_in(j, S::R1))
+          a[j] = B[col_pos<L, PAIRS>(lt + S::R2 * half_row(j, S::R1), cl)];
+        continue;
+      }
       const int r = (lt + S::R2 * j + in_add) & (L - 1);
       a[j] = r < in_count ? B[col_pos<L, PAIRS>(r, cl)] : make_float2(0.f, 0.f);
     }
-    reg_fft<S::R1, Rm<L>::V, INV>(a, w);
-    const int rho = (lt + in_add) & (S::R2 - 1);
+    reg_fft<S::R1, Rm<L>::V, INV, HALF && !INV>(a, w);
+    // (HALF: in_add = L / 4, a multiple of R2; the inverse has in_add 0)
+    const int rho = HALF ? lt : (lt + in_add) & (S::R2 - 1);
 #pragma unroll
     for (int k1 = 0; k1 < S::R1; ++k1)
     {
       float2 v = a[k1];
       if (k1 != 0)
       {
-        float2 r = tw[(lt * k1) & (L - 1)];
+        float2 r = tw[lt * k1];
         if (INV)
           r.y = -r.y;
         v = cmul(v, r);
@@ -177,8 +199,8 @@ __device__ __forceinline__ void col_tile_fft(float2 *B, int cl, int lt,
   {
 #pragma unroll
     for (int u = 0; u < S::R2; ++u)
-      b[u] = B[col_pos<L, PAIRS>(lt * S::R2 + ((u + in_add) & (S::R2 - 1)),
-                                  cl)];
+      b[u] = B[col_pos<L, PAIRS>(
+          lt * S::R2 + (HALF ? u : ((u + in_add) & (S::R2 - 1))), cl)];
     reg_fft<S::R2, Rm<L>::V, INV>(b, w);
   }
 }
@@ -186,7 +208,7 @@ __device__ __forceinline__ void col_tile_fft(float2 *B, int cl, int lt,
 // The same transform for two adjacent columns 2 cp, 2 cp + 1 of a tile of
 // TC-column rows (one 16-byte shared access per row and stage for both,
 // one twiddle load for both).  Outputs k = lt + R1 * k2 in b0 / b1.
-template <int L, bool INV>
+template <int L, bool INV, bool HALF>
 __device__ __forceinline__ void col_tile_fft2(float2 *B, int cp, int lt,
                                               int in_add, int in_count,
                                               const float2 (&w)[Rm<L>::V / 2],
@@ -203,22 +225,32 @@ __device__ __forceinline__ void col_tile_fft2(float2 *B, int cp, int lt,
 #pragma unroll
     for (int j = 0; j < S::R1; ++j)
     {
+      if (HALF && !INV)
+      {
+        if (half_in(j, S::R1))
+        {
+          const float4 v = B4[(lt + S::R2 * half_row(j, S::R1)) * TP + cp];
+          a0[j] = make_float2(v.x, v.y);
+          a1[j] = make_float2(v.z, v.w);
+        }
+        continue;
+      }
       const int r = (lt + S::R2 * j + in_add) & (L - 1);
       const float4 v =
           r < in_count ? B4[r * TP + cp] : make_float4(0.f, 0.f, 0.f, 0.f);
       a0[j] = make_float2(v.x, v.y);
       a1[j] = make_float2(v.z, v.w);
     }
-    reg_fft<S::R1, Rm<L>::V, INV>(a0, w);
-    reg_fft<S::R1, Rm<L>::V, INV>(a1, w);
-    const int rho = (lt + in_add) & (S::R2 - 1);
+    reg_fft<S::R1, Rm<L>::V, INV, HALF && !INV>(a0, w);
+    reg_fft<S::R1, Rm<L>::V, INV, HALF && !INV>(a1, w);
+    const int rho = HALF ? lt : (lt + in_add) & (S::R2 - 1);
 #pragma unroll
     for (int k1 = 0; k1 < S::R1; ++k1)
     {
       float2 v0 = a0[k1], v1 = a1[k1];
       if (k1 != 0)
       {
-        float2 r = tw[(lt * k1) & (L - 1)];
+        float2 r = tw[lt * k1];
         if (INV)
           r.y = -r.y;
         v0 = cmul(v0, r);
@@ -234,7 +266,8 @@ __device__ __forceinline__ void col_tile_fft2(float2 *B, int cp, int lt,
     for (int u = 0; u < S::R2; ++u)
     {
       const float4 v =
-          B4[(lt * S::R2 + ((u + in_add) & (S::R2 - 1))) * TP + cp];
+          B4[(lt * S::R2 + (HALF ? u : ((u + in_add) & (S::R2 - 1)))) * TP +
+             cp];
       b0[u] = make_float2(v.x, v.y);
       b1[u] = make_float2(v.z, v.w);
     }
@@ -261,7 +294,7 @@ __device__ __forceinline__ void col_tile_fft2(float2 *B, int cp, int lt,
 // covers an odd last coil (pair tail_pl) with a one-coil map whose second
 // coil is out of range (zero fill).  CPT 2 (PAIRED 2 only): each thread
 // runs two adjacent columns of one coil (col_tile_fft2), half the threads.
-template <int L, bool INV, int PAIRED, int CPT = 1>
+template <int L, bool INV, int PAIRED, int CPT = 1, bool HALF = false>
 __global__ void __launch_bounds__(Shape<L>::CT / CPT, 3)
     k_fft_cols_tma(const __grid_constant__ CUtensorMap tmap,
                    const __grid_constant__ CUtensorMap tail, long long tail_pl,
@@ -372,14 +405,22 @@ __global__ void __launch_bounds__(Shape<L>::CT / CPT, 3)
         cr = __ldg(colrange + col);
       const bool on = col < ncols && cr.x <= cr.y;
       float2 bv[S::R2];
-      col_tile_fft<L, INV, PAIRED == 1>(buf + (size_t)b * L * TC, cl, lt,
-                                        in_add, in_count, w, tw, bv);
+      col_tile_fft<L, INV, PAIRED == 1, HALF>(buf + (size_t)b * L * TC, cl,
+                                              lt, in_add, in_count, w, tw, bv);
       if (lt < S::R1 && on)
       {
 #pragma unroll
         for (int k2 = 0; k2 < S::R2; ++k2)
         {
-          const int r = (lt + S::R1 * k2 + out_add) & (L - 1);
+          if (HALF && INV)
+          {
+            if (half_in(k2, S::R2))
+              dp[(long long)(lt + S::R1 * half_row(k2, S::R2)) * rs] = bv[k2];
+            continue;
+          }
+          // (HALF forward: out_add = L / 2)
+          const int r = HALF ? lt + S::R1 * ((k2 + S::R2 / 2) % S::R2)
+                             : (lt + S::R1 * k2 + out_add) & (L - 1);
           if (r < out_count && (unsigned)r >= cr.x && (unsigned)r <= cr.y)
             dp[(long long)r * rs] = bv[k2];
         }
@@ -394,14 +435,16 @@ __global__ void __launch_bounds__(Shape<L>::CT / CPT, 3)
         cr1 = __ldg(colrange + col + 1);
       }
       float2 b0[S::R2], b1[S::R2];
-      col_tile_fft2<L, INV>(buf + (size_t)b * L * TC, cl, lt, in_add,
-                            in_count, w, tw, b0, b1);
+      static_assert(!(HALF && INV), "coil pairs are forward only");
+      col_tile_fft2<L, INV, HALF>(buf + (size_t)b * L * TC, cl, lt, in_add,
+                                  in_count, w, tw, b0, b1);
       if (lt < S::R1 && col < ncols)
       {
 #pragma unroll
         for (int k2 = 0; k2 < S::R2; ++k2)
         {
-          const int r = (lt + S::R1 * k2 + out_add) & (L - 1);
+          const int r = HALF ? lt + S::R1 * ((k2 + S::R2 / 2) % S::R2)
+                             : (lt + S::R1 * k2 + out_add) & (L - 1);
           if (r < out_count && (unsigned)r >= cr0.x && (unsigned)r <= cr0.y)
             dp[(long long)r * rs] = b0[k2];
           if (r < out_count && (unsigned)r >= cr1.x && (unsigned)r <= cr1.y)
@@ -425,7 +468,7 @@ __global__ void __launch_bounds__(Shape<L>::CT / CPT, 3)
 // conj(S) coil sum in coil order (or per-coil outputs).  src: coil c,
 // row r, column col at c * coil_stride + r * ncols + col; image pixel of
 // output row n and column col: n * ncols + col.
-template <int L, bool SENS>
+template <int L, bool SENS, bool HALF>
 __global__ void __launch_bounds__(Shape<L>::CT, L <= 256 ? 3 : 1)
     k_fft_cols_sum(const float2 *__restrict__ src, long long ncols,
                    long long coil_stride, const float *__restrict__ deapo,
@@ -473,8 +516,11 @@ __global__ void __launch_bounds__(Shape<L>::CT, L <= 256 ? 3 : 1)
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
       {
-        const int n = (lt + S::R1 * k2 + out_add) & (L - 1);
-        if (n >= n_out)
+        if (HALF && !half_in(k2, S::R2))
+          continue;
+        const int n = HALF ? lt + S::R1 * half_row(k2, S::R2)
+                           : (lt + S::R1 * k2 + out_add) & (L - 1);
+        if (!HALF && n >= n_out)
           continue;
         const long long px = (long long)n * ncols + col;
         // crop -> FFT scaling -> deapodization (gpuNUFFT_operator.cpp:
@@ -505,8 +551,11 @@ __global__ void __launch_bounds__(Shape<L>::CT, L <= 256 ? 3 : 1)
 #pragma unroll
     for (int k2 = 0; k2 < S::R2; ++k2)
     {
-      const int n = (lt + S::R1 * k2 + out_add) & (L - 1);
-      if (n >= n_out)
+      if (HALF && !half_in(k2, S::R2))
+        continue;
+      const int n = HALF ? lt + S::R1 * half_row(k2, S::R2)
+                         : (lt + S::R1 * k2 + out_add) & (L - 1);
+      if (!HALF && n >= n_out)
         continue;
       const long long px = (long long)n * ncols + col;
       if (partial)
@@ -549,7 +598,7 @@ template <int L> struct SumTma
   }
 };
 
-template <int L>
+template <int L, bool HALF>
 __global__ void __launch_bounds__(Shape<L>::CT, 2)
     k_fft_cols_sum_tma(const __grid_constant__ CUtensorMap src_map,
                        const __grid_constant__ CUtensorMap sens_map,
@@ -654,14 +703,17 @@ __global__ void __launch_bounds__(Shape<L>::CT, 2)
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
       {
-        const int n = (lt + S::R1 * k2 + out_add) & (L - 1);
+        if (HALF && !half_in(k2, S::R2))
+          continue;
+        const int n = HALF ? lt + S::R1 * half_row(k2, S::R2)
+                           : (lt + S::R1 * k2 + out_add) & (L - 1);
         d[k2] = (on && n < n_out) ? __ldg(deapo + (long long)n * ncols + col)
                                   : 0.f;
         acc[k2] = make_float2(0.f, 0.f);
       }
     }
     float2 bv[S::R2];
-    col_tile_fft<L, true, false>(src_t + (size_t)b * L * TC, cl, lt, 0, L, w,
+    col_tile_fft<L, true, false, HALF>(src_t + (size_t)b * L * TC, cl, lt, 0, L, w,
                                  tw, bv);
     if (on)
     {
@@ -669,8 +721,11 @@ __global__ void __launch_bounds__(Shape<L>::CT, 2)
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
       {
-        const int n = (lt + S::R1 * k2 + out_add) & (L - 1);
-        if (n >= n_out)
+        if (HALF && !half_in(k2, S::R2))
+          continue;
+        const int n = HALF ? lt + S::R1 * half_row(k2, S::R2)
+                           : (lt + S::R1 * k2 + out_add) & (L - 1);
+        if (!HALF && n >= n_out)
           continue;
         // crop -> FFT scaling -> deapodization -> conj(S) * v, running coil
         // sum (gpuNUFFT_operator.cpp:800-819, std_gpuNUFFT_kernels.cu:
@@ -695,8 +750,11 @@ __global__ void __launch_bounds__(Shape<L>::CT, 2)
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
       {
-        const int n = (lt + S::R1 * k2 + out_add) & (L - 1);
-        if (n >= n_out)
+        if (HALF && !half_in(k2, S::R2))
+          continue;
+        const int n = HALF ? lt + S::R1 * half_row(k2, S::R2)
+                           : (lt + S::R1 * k2 + out_add) & (L - 1);
+        if (!HALF && n >= n_out)
           continue;
         const long long px = (long long)n * ncols + col;
         if (partial)
@@ -746,7 +804,7 @@ __global__ void k_sum_coil_groups(const float2 *__restrict__ partial,
 // One line per (image row, coil), coil fastest: a block's lines share image
 // rows, so the image is read once per block.  Output A[c][row][k],
 // rows = N_y * N_z.
-template <int L, bool SENS>
+template <int L, bool SENS, bool HALF>
 __global__ void __launch_bounds__(kFftThreads, L <= 256 ? 4 : 1)
     k_fft_rows_fwd(const float2 *__restrict__ image,
                    const float2 *__restrict__ sens,
@@ -775,9 +833,12 @@ __global__ void __launch_bounds__(kFftThreads, L <= 256 ? 4 : 1)
 #pragma unroll
     for (int j = 0; j < S::R1; ++j)
     {
-      const int xp = (lt + S::R2 * j + in_add) & (L - 1);
+      if (HALF && !half_in(j, S::R1))
+        continue;
+      const int xp = HALF ? lt + S::R2 * half_row(j, S::R1)
+                          : (lt + S::R2 * j + in_add) & (L - 1);
       float2 v = make_float2(0.f, 0.f);
-      if (on && xp < Nx)
+      if (on && (HALF || xp < Nx))
       {
         const long long px = rbase + xp;
         if (SENS)
@@ -794,7 +855,7 @@ __global__ void __launch_bounds__(kFftThreads, L <= 256 ? 4 : 1)
       }
       a[j] = v;
     }
-    stage1<L, false, 1>(a, lt, w, tw, Y);
+    stage1<L, false, 1, HALF>(a, lt, w, tw, Y);
   }
   __syncthreads();
   if (lt < S::R1 && on)
@@ -804,7 +865,8 @@ __global__ void __launch_bounds__(kFftThreads, L <= 256 ? 4 : 1)
     float2 *out = A + ((long long)c * rows + row) * L;
 #pragma unroll
     for (int k2 = 0; k2 < S::R2; ++k2)
-      out[(lt + S::R1 * k2 + out_add) & (L - 1)] = b[k2];
+      out[HALF ? lt + S::R1 * ((k2 + S::R2 / 2) % S::R2)
+               : (lt + S::R1 * k2 + out_add) & (L - 1)] = b[k2];
   }
 }
 
@@ -839,7 +901,7 @@ struct RowsTma
   }
 };
 
-template <int L, bool SENS>
+template <int L, bool SENS, bool HALF>
 __global__ void __launch_bounds__(kFftThreads, 3)
     k_fft_rows_fwd_tma(const __grid_constant__ CUtensorMap coil_map,
                        const float2 *__restrict__ image,
@@ -928,9 +990,12 @@ __global__ void __launch_bounds__(kFftThreads, 3)
 #pragma unroll
       for (int q = 0; q < S::R1; ++q)
       {
-        const int xp = (lt + S::R2 * q + in_add) & (L - 1);
+        if (HALF && !half_in(q, S::R1))
+          continue;
+        const int xp = HALF ? lt + S::R2 * half_row(q, S::R1)
+                            : (lt + S::R2 * q + in_add) & (L - 1);
         float2 v = make_float2(0.f, 0.f);
-        if (xp < Nx)
+        if (HALF || xp < Nx)
         {
           if (SENS)
           {  // sensMulKernel, then deapodization (std_gpuNUFFT_kernels.cu)
@@ -946,7 +1011,7 @@ __global__ void __launch_bounds__(kFftThreads, 3)
         }
         a[q] = v;
       }
-      stage1<L, false, 1>(a, lt, w, tw, Y);
+      stage1<L, false, 1, HALF>(a, lt, w, tw, Y);
     }
     __syncthreads();  // stage b read; exchange written
     if (threadIdx.x == 0 && j + 2 * stride < n_jobs)
@@ -958,7 +1023,8 @@ __global__ void __launch_bounds__(kFftThreads, 3)
       float2 *out = A + ((long long)c * rows + row) * L;
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
-        out[(lt + S::R1 * k2 + out_add) & (L - 1)] = bv[k2];
+        out[HALF ? lt + S::R1 * ((k2 + S::R2 / 2) % S::R2)
+                 : (lt + S::R1 * k2 + out_add) & (L - 1)] = bv[k2];
     }
   }
 }
@@ -1164,6 +1230,15 @@ template <class F> void with_length(int L, F &&f)
   }
 }
 
+// f(true_type / false_type): the kernels for axes oversampled by two
+template <class F> void with_half(bool half, F &&f)
+{
+  if (half)
+    f(std::true_type());
+  else
+    f(std::false_type());
+}
+
 template <class K> void set_smem(K kernel, size_t bytes)
 {
   if (bytes > 48 * 1024)
@@ -1264,6 +1339,11 @@ void cols(int L, const float2 *src, float2 *dst, long long ncols,
           const uint32_t *tiles = nullptr, long long n_list = 0,
           int list_cols = 0)
 {
+  // the HALF kernels' row maps (fftcore::half_in)
+  const bool half = INV ? in_add == 0 && in_count == L && out_add == L / 4 &&
+                              out_count == L / 2 && !colrange
+                        : in_add == L / 4 && in_count == L / 2 &&
+                              out_add == L / 2 && out_count == L;
   bool done = false;
   if (!pow2_length(L))
   {
@@ -1330,12 +1410,15 @@ void cols(int L, const float2 *src, float2 *dst, long long ncols,
         // bound by instruction issue) runs two adjacent columns per thread;
         // the plain passes, closer to the DRAM bound, keep the warps of one
         // column per thread
-        if (mode == 2)
-          launch(k_fft_cols_tma<LL, INV, 2, 2>, S::CT / 2);
-        else if (mode == 1)
-          launch(k_fft_cols_tma<LL, INV, 1>, S::CT);
-        else
-          launch(k_fft_cols_tma<LL, INV, 0>, S::CT);
+        with_half(half, [&](auto hc) {
+          constexpr bool H = decltype(hc)::value;
+          if (mode == 2)
+            launch(k_fft_cols_tma<LL, INV, 2, 2, H && !INV>, S::CT / 2);
+          else if (mode == 1)
+            launch(k_fft_cols_tma<LL, INV, 1>, S::CT);
+          else  // (256: at the DRAM rate either way, and slower with HALF)
+            launch(k_fft_cols_tma<LL, INV, 0, 1, H && LL < 256>, S::CT);
+        });
         GN_LAUNCH_CHECK("pruned column transform (tensor-copy tiles)");
         done = true;
       }
@@ -1347,7 +1430,7 @@ void cols(int L, const float2 *src, float2 *dst, long long ncols,
   with_length(L, [&](auto lc) {
     constexpr int LL = decltype(lc)::value;
     using S = Shape<LL>;
-    auto k = k_fft_cols<LL, INV>;
+    auto k = half ? k_fft_cols<LL, INV, true> : k_fft_cols<LL, INV, false>;
     set_smem(k, S::col_smem());
     if (planes > 65535)
       throw Error(kNotSupported, "too many planes for the pruned transform");
@@ -1391,7 +1474,8 @@ bool launch_cols_sum_tma(const float2 *src, long long ncols,
     if (cudaGetDevice(&dev) == cudaSuccess)
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long blocks = n_units < 2LL * sms ? n_units : 2LL * sms;
-    auto k = k_fft_cols_sum_tma<L>;
+    const bool half = n_out == L / 2 && out_add == L / 4;
+    auto k = half ? k_fft_cols_sum_tma<L, true> : k_fft_cols_sum_tma<L, false>;
     set_smem(k, smem);
     k<<<(unsigned)blocks, S::CT, smem, s>>>(
         src_map, sens_map, ncols, (int)n_units, FastDiv((uint32_t)groups),
@@ -1460,10 +1544,14 @@ bool launch_rows_fwd_tma(const float2 *image, const float2 *sens,
           tm, image, deapo, Nx, rows, C, (int)n_jobs, FastDiv((uint32_t)n_cc),
           in_add, out_add, roots, A, cw);
     };
-    if (sens)
-      launch(k_fft_rows_fwd_tma<L, true>);
-    else
-      launch(k_fft_rows_fwd_tma<L, false>);
+    with_half(Nx == L / 2 && in_add == L / 4 && out_add == L / 2,
+              [&](auto hc) {
+                constexpr bool H = decltype(hc)::value;
+                if (sens)
+                  launch(k_fft_rows_fwd_tma<L, true, H>);
+                else
+                  launch(k_fft_rows_fwd_tma<L, false, H>);
+              });
     GN_LAUNCH_CHECK("pruned forward rows (tensor-copy tiles)");
     return true;
   }
@@ -1536,22 +1624,16 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
     if (launch_rows_fwd_tma<LL>(image, sens, deapo, g.N[0], rows, N, C,
                                 in_add, out_add, roots[0], tmp_a, cw, s))
       return;
-    if (sens)
-    {
-      auto k = k_fft_rows_fwd<LL, true>;
-      set_smem(k, S::smem());
-      k<<<(unsigned)nb, kFftThreads, S::smem(), s>>>(
-          image, sens, deapo, g.N[0], rows, N, C, in_add, out_add, roots[0],
-          tmp_a);
-    }
-    else
-    {
-      auto k = k_fft_rows_fwd<LL, false>;
-      set_smem(k, S::smem());
-      k<<<(unsigned)nb, kFftThreads, S::smem(), s>>>(
-          image, sens, deapo, g.N[0], rows, N, C, in_add, out_add, roots[0],
-          tmp_a);
-    }
+    with_half(g.N[0] == LL / 2 && in_add == LL / 4 && out_add == LL / 2,
+              [&](auto hc) {
+                constexpr bool H = decltype(hc)::value;
+                auto k = sens ? k_fft_rows_fwd<LL, true, H>
+                              : k_fft_rows_fwd<LL, false, H>;
+                set_smem(k, S::smem());
+                k<<<(unsigned)nb, kFftThreads, S::smem(), s>>>(
+                    image, sens, deapo, g.N[0], rows, N, C, in_add, out_add,
+                    roots[0], tmp_a);
+              });
     GN_LAUNCH_CHECK("pruned forward rows");
   });
   // y: A -> (3-D) B [C][N_z][G_y][G_x] or (2-D) the grid
@@ -1675,6 +1757,7 @@ void launch_pruned_adjoint_xfirst(const float2 *xrows, const float *deapo,
     constexpr int LL = decltype(lc)::value;
     using S = Shape<LL>;
     const long long nb = (ncols + S::TC - 1) / S::TC;
+    const bool half = g.N[ax] == LL / 2 && out_add == LL / 4;
     split_coils(nb);
     const dim3 grd((unsigned)nb, (unsigned)groups);
     const bool tiles =
@@ -1684,7 +1767,8 @@ void launch_pruned_adjoint_xfirst(const float2 *xrows, const float *deapo,
                                            roots[ax], out, partial, cw, s);
     if (combine && !tiles)
     {
-      auto k = k_fft_cols_sum<LL, true>;
+      auto k = half ? k_fft_cols_sum<LL, true, true>
+                    : k_fft_cols_sum<LL, true, false>;
       set_smem(k, S::col_smem());
       k<<<grd, S::CT, S::col_smem(), s>>>(src, ncols, coil_stride, deapo,
                                          sens, g.N[ax], N, C, cpb, out_add,
@@ -1693,7 +1777,8 @@ void launch_pruned_adjoint_xfirst(const float2 *xrows, const float *deapo,
     }
     else if (!combine)
     {
-      auto k = k_fft_cols_sum<LL, false>;
+      auto k = half ? k_fft_cols_sum<LL, false, true>
+                    : k_fft_cols_sum<LL, false, false>;
       set_smem(k, S::col_smem());
       k<<<grd, S::CT, S::col_smem(), s>>>(src, ncols, coil_stride, deapo,
                                          nullptr, g.N[ax], N, C, cpb, out_add,
