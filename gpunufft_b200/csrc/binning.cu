@@ -455,7 +455,8 @@ namespace
 // Range of z (grid cells with at least one interpolation weight) per (y, x)
 // column, widened by one cell each way; empty columns keep lo > hi.
 __global__ void k_col_ranges(const uint32_t *__restrict__ row_off, int G0,
-                             int G1, int G2, uint2 *__restrict__ range)
+                             int G1, int G2, int x_shift,
+                             uint2 *__restrict__ range)
 {
   const long long n = (long long)G0 * G1 * G2;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n;
@@ -463,7 +464,9 @@ __global__ void k_col_ranges(const uint32_t *__restrict__ row_off, int G0,
   {
     if (row_off[c + 1] == row_off[c])
       continue;
-    const long long col = c % ((long long)G0 * G1);
+    long long col = c % ((long long)G0 * G1);
+    const int x = (int)(col % G0);
+    col += x + x_shift < G0 ? x_shift : x_shift - G0;  // its stored column
     const int z = (int)(c / ((long long)G0 * G1));
     atomicMin(&range[col].x, (unsigned)max(z - 1, 0));
     atomicMax(&range[col].y, (unsigned)min(z + 1, G2 - 1));
@@ -471,7 +474,7 @@ __global__ void k_col_ranges(const uint32_t *__restrict__ row_off, int G0,
 }
 }  // namespace
 
-void build_column_ranges(const uint32_t *row_off, const Geo &g,
+void build_column_ranges(const uint32_t *row_off, const Geo &g, int x_shift,
                          DeviceBuffer &range, DeviceBuffer &tiles,
                          int &n_tiles, cudaStream_t s)
 {
@@ -481,7 +484,7 @@ void build_column_ranges(const uint32_t *row_off, const Geo &g,
   GN_CUDA(cudaMemcpyAsync(range.get(), h.data(), cols * sizeof(uint2),
                           cudaMemcpyHostToDevice, s));
   k_col_ranges<<<grid_for(g.grid_count, 256, 148 * 64), 256, 0, s>>>(
-      row_off, g.G[0], g.G[1], g.G[2], range.as<uint2>());
+      row_off, g.G[0], g.G[1], g.G[2], x_shift, range.as<uint2>());
   GN_LAUNCH_CHECK("column ranges");
   GN_CUDA(cudaMemcpyAsync(h.data(), range.get(), cols * sizeof(uint2),
                           cudaMemcpyDeviceToHost, s));

@@ -71,8 +71,9 @@ size_t build_interp_matrix(const float *traj_sorted,
 // `tiles` lists (ascending, n_tiles of them) the tiles of kColTile adjacent
 // columns (tile t: columns t * kColTile ...) that hold at least one range;
 // the forward z pass transforms only those.
+// Cell x is stored at x + x_shift mod G (columns are counted as stored).
 constexpr int kColTile = 8;
-void build_column_ranges(const uint32_t *row_off, const Geo &g,
+void build_column_ranges(const uint32_t *row_off, const Geo &g, int x_shift,
                          DeviceBuffer &range, DeviceBuffer &tiles,
                          int &n_tiles, cudaStream_t s);
 

@@ -865,8 +865,7 @@ __global__ void __launch_bounds__(kFftThreads, L <= 256 ? 4 : 1)
     float2 *out = A + ((long long)c * rows + row) * L;
 #pragma unroll
     for (int k2 = 0; k2 < S::R2; ++k2)
-      out[HALF ? lt + S::R1 * ((k2 + S::R2 / 2) % S::R2)
-               : (lt + S::R1 * k2 + out_add) & (L - 1)] = b[k2];
+      out[(lt + S::R1 * k2 + out_add) & (L - 1)] = b[k2];
   }
 }
 
@@ -1023,8 +1022,7 @@ __global__ void __launch_bounds__(kFftThreads, 3)
       float2 *out = A + ((long long)c * rows + row) * L;
 #pragma unroll
       for (int k2 = 0; k2 < S::R2; ++k2)
-        out[HALF ? lt + S::R1 * ((k2 + S::R2 / 2) % S::R2)
-                 : (lt + S::R1 * k2 + out_add) & (L - 1)] = bv[k2];
+        out[(lt + S::R1 * k2 + out_add) & (L - 1)] = bv[k2];
     }
   }
 }
@@ -1544,7 +1542,7 @@ bool launch_rows_fwd_tma(const float2 *image, const float2 *sens,
           tm, image, deapo, Nx, rows, C, (int)n_jobs, FastDiv((uint32_t)n_cc),
           in_add, out_add, roots, A, cw);
     };
-    with_half(Nx == L / 2 && in_add == L / 4 && out_add == L / 2,
+    with_half(Nx == L / 2 && in_add == L / 4,
               [&](auto hc) {
                 constexpr bool H = decltype(hc)::value;
                 if (sens)
@@ -1603,7 +1601,7 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
                            float2 *tmp_b, float2 *grid, cudaStream_t s,
                            const uint2 *zrange, tma::CopyWait cw,
                            bool paired, const uint32_t *ztiles, int n_ztiles,
-                           int ztile_cols)
+                           int ztile_cols, int x_shift)
 {
   const long long N = g.img_count;
   const long long rows = (long long)g.N[1] * g.N[2];
@@ -1611,7 +1609,8 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
   if (!pow2_length(g.G[0]))
     gen_rows_fwd(g.G[0], image, sens, deapo, g.N[0], rows, N, C,
                  pos_mod((long long)g.shift_inv[0] - g.crop[0], g.G[0]),
-                 pos_mod(-(long long)g.shift_fwd[0], g.G[0]), roots[0], tmp_a,
+                 pos_mod(x_shift - (long long)g.shift_fwd[0], g.G[0]),
+                 roots[0], tmp_a,
                  s);
   else
   with_length(g.G[0], [&](auto lc) {
@@ -1620,11 +1619,12 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
     const long long nb = (rows * C + S::NL - 1) / S::NL;
     const int in_add = pos_mod((long long)g.shift_inv[0] - g.crop[0], g.G[0]);
     // the FORWARD fftshift: frequency k is stored at (k - ceil(G/2)) mod G
-    const int out_add = pos_mod(-(long long)g.shift_fwd[0], g.G[0]);
+    const int out_add =
+        pos_mod(x_shift - (long long)g.shift_fwd[0], g.G[0]);
     if (launch_rows_fwd_tma<LL>(image, sens, deapo, g.N[0], rows, N, C,
                                 in_add, out_add, roots[0], tmp_a, cw, s))
       return;
-    with_half(g.N[0] == LL / 2 && in_add == LL / 4 && out_add == LL / 2,
+    with_half(g.N[0] == LL / 2 && in_add == LL / 4,
               [&](auto hc) {
                 constexpr bool H = decltype(hc)::value;
                 auto k = sens ? k_fft_rows_fwd<LL, true, H>

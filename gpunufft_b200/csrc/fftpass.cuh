@@ -57,7 +57,8 @@ size_t pruned_scratch_b(const Geo &g, int C);
 // cell q of coil c at ((c / 2) * G + q) * 2 + c % 2 (C rounded up to even
 // coils of storage).  ztiles (paired only): the n_ztiles column tiles of
 // ztile_cols columns (ascending) that hold a z range; the z pass transforms
-// only these (the others have no cell the interpolation reads).
+// only these (the others have no cell the interpolation reads).  x_shift:
+// cell x is stored at x + x_shift mod G (zrange and ztiles as stored).
 void launch_pruned_forward(const float2 *image, const float2 *sens,
                            const float *deapo, const Geo &g, int C,
                            const float2 *const roots[3], float2 *tmp_a,
@@ -66,7 +67,7 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
                            tma::CopyWait cw = tma::CopyWait(),
                            bool paired = false,
                            const uint32_t *ztiles = nullptr, int n_ztiles = 0,
-                           int ztile_cols = 0);
+                           int ztile_cols = 0, int x_shift = 0);
 
 // Adjoint: grid [C][G] (INVERSE fftshift folded in by the adjoint spread)
 // -> unnormalised inverse DFT -> crop of the second INVERSE fftshift ->

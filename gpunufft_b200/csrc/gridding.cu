@@ -217,13 +217,10 @@ __device__ __forceinline__ int compact_axis(float c, int ax, int sec_ax,
     imax = pmax;
   if (imin >= pmax)
     imin = (int)(pmax - 2 * g.kernel_radius);
-  int n = 0;
-#pragma unroll
-  for (int k = 0; k < KS; ++k)
-  {
-    li[k] = 0;
-    w[k] = 0.0f;
-  }
+  // the valid candidates are consecutive (d^2 grows away from the sample):
+  // their mask gives the first and the count, and the weights move down to
+  // slot 0 by the bits of the first
+  unsigned mask = 0;
 #pragma unroll
   for (int k = 0; k < KS; ++k)
   {
@@ -233,26 +230,32 @@ __device__ __forceinline__ int compact_axis(float c, int ax, int sec_ax,
     const float d = __fmul_rn(__fsub_rn(kx, c), g.aniso[ax]);
     const float d2 = __fmul_rn(d, d);
     bool valid = i <= imax && i >= 0;
-    float wt;
     if (g.texture)
-      wt = texture_weight(g, lut, __fmul_rn(d2, g.radius_sq_inv));
+    {
+      const float wt = texture_weight(g, lut, __fmul_rn(d2, g.radius_sq_inv));
+      w[k] = valid ? wt : 0.0f;
+    }
     else
     {
       valid = valid && d2 < g.radius_sq;
       int lx = (int)roundf(__fmul_rn(d2, g.dist_mult));
       lx = lx < 0 ? 0 : (lx > g.lut_len - 1 ? g.lut_len - 1 : lx);
-      wt = valid ? __ldg(lut + lx) : 0.0f;
+      w[k] = valid ? __ldg(lut + lx) : 0.0f;
     }
-    // append (static indices only: entry j receives candidate k if j == n)
-#pragma unroll
-    for (int j = 0; j < KS; ++j)
-      if (valid && j == n)
-      {
-        li[j] = i;
-        w[j] = wt;
-      }
-    n += valid ? 1 : 0;
+    mask |= valid ? 1u << k : 0u;
   }
+  const int n = __popc(mask), first = n ? __ffs(mask) - 1 : 0;
+#pragma unroll
+  for (int s = 1; s < KS; s <<= 1)
+    if (first & s)
+    {
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+        w[k] = k + s < KS ? w[k + s] : 0.0f;
+    }
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+    li[k] = n ? imin + first + k : 0;
   return n;
 }
 
@@ -1135,76 +1138,101 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
   }
 
-  for (int t = it.begin + threadIdx.x; t < it.end; t += kThreads)
-  {
-    int l[3][KS];
-    float w[3][KS];
-    int n[3] = {1, 1, 1};
-    l[2][0] = 0;
-    w[2][0] = 1.f;
-#pragma unroll
-    for (int a = 0; a < DIM; ++a)
-      n[a] = compact_axis<KS>(__ldg(traj + (size_t)a * M + t), a, sa[a], g,
-                              lut, l[a], w[a]);
-    float2 acc[CG];
-#pragma unroll
-    for (int c = 0; c < CG; ++c)
-      acc[c] = make_float2(0.f, 0.f);
-    // tile-frame entries are consecutive cells starting at l[a][0]
-    const int xb = l[0][0] + dx;
-    for (int z = 0; z < n[2]; ++z)
+  // Items of few samples split the tile's coils over the threads: PARTS
+  // threads per sample, CG / PARTS coils each -- at least MINC, since every
+  // thread computes its sample's footprint.  2-D 256^2 x 16, 103 k radial
+  // samples (25 per sector): 71 us with a thread per sample, 47 us so; 320^2
+  // x 8, kernel width 4: 46 -> 37 us with 6 footprint slots.
+  constexpr int MINC = KS == 4 ? 1 : 2;
+  const int n_samples = it.end - it.begin;
+  auto run = [&](auto ptc) {
+    constexpr int PARTS = decltype(ptc)::value, CT = CG / PARTS;
+    constexpr int PER = kThreads / PARTS;  // samples at a time
+    const int first = PARTS > 1 ? (int)(threadIdx.x / PER) * CT : 0;
+    const float2 *tp = tile + first * cstride;
+    for (int t = it.begin + (int)(threadIdx.x % PER); t < it.end; t += PER)
     {
-      float wzv = 1.f;
+      int l[3][KS];
+      float w[3][KS];
+      int n[3] = {1, 1, 1};
+      l[2][0] = 0;
+      w[2][0] = 1.f;
 #pragma unroll
-      for (int k = 0; k < KS; ++k)
-        if (k == z)
-          wzv = w[2][k];
-      for (int y = 0; y < n[1]; ++y)
+      for (int a = 0; a < DIM; ++a)
+        n[a] = compact_axis<KS>(__ldg(traj + (size_t)a * M + t), a, sa[a], g,
+                                lut, l[a], w[a]);
+      float2 acc[CT];
+#pragma unroll
+      for (int c = 0; c < CT; ++c)
+        acc[c] = make_float2(0.f, 0.f);
+      // tile-frame entries are consecutive cells starting at l[a][0]
+      const int xb = l[0][0] + dx;
+      for (int z = 0; z < n[2]; ++z)
       {
-        float wyv = 0.f;
+        float wzv = 1.f;
 #pragma unroll
         for (int k = 0; k < KS; ++k)
-          if (k == y)
-            wyv = w[1][k];
-        const float wzy = DIM == 3 ? __fmul_rn(wzv, wyv) : wyv;
-        const int row = ((DIM == 3 ? (l[2][0] + z) * PY : 0) + l[1][0] + y) *
-                            PX + xb;
-#pragma unroll
-        for (int x = 0; x < KS; ++x)
+          if (k == z)
+            wzv = w[2][k];
+        for (int y = 0; y < n[1]; ++y)
         {
-          if (x < n[0])
-          {
-            const float wt = __fmul_rn(wzy, w[0][x]);
+          float wyv = 0.f;
 #pragma unroll
-            for (int c = 0; c < CG; ++c)
+          for (int k = 0; k < KS; ++k)
+            if (k == y)
+              wyv = w[1][k];
+          const float wzy = DIM == 3 ? __fmul_rn(wzv, wyv) : wyv;
+          const int row =
+              ((DIM == 3 ? (l[2][0] + z) * PY : 0) + l[1][0] + y) * PX + xb;
+#pragma unroll
+          for (int x = 0; x < KS; ++x)
+          {
+            if (x < n[0])
             {
-              const float2 v = tile[c * cstride + row + x];
-              acc[c].x = __fmaf_rn(v.x, wt, acc[c].x);
-              acc[c].y = __fmaf_rn(v.y, wt, acc[c].y);
+              const float wt = __fmul_rn(wzy, w[0][x]);
+#pragma unroll
+              for (int c = 0; c < CT; ++c)
+              {
+                const float2 v = tp[c * cstride + row + x];
+                acc[c].x = __fmaf_rn(v.x, wt, acc[c].x);
+                acc[c].y = __fmaf_rn(v.y, wt, acc[c].y);
+              }
             }
           }
         }
       }
-    }
-    const uint32_t j = __ldg(idx + t);
-    const float sd = dens ? sqrtf(__ldg(dens + t)) : 1.0f;
+      const uint32_t j = __ldg(idx + t);
+      const float sd = dens ? sqrtf(__ldg(dens + t)) : 1.0f;
 #pragma unroll
-    for (int c = 0; c < CG; ++c)
-    {
-      if (c0 + c < C)
+      for (int c = 0; c < CT; ++c)
       {
-        // performFFTScaling then performDensityCompensation
-        // (std_gpuNUFFT_kernels.cu:114-140, 220-242)
-        float ax = __fmul_rn(acc[c].x, scale), ay = __fmul_rn(acc[c].y, scale);
-        if (dens)
+        const int cc = c0 + first + c;
+        if (cc < C)
         {
-          ax = __fmul_rn(ax, sd);
-          ay = __fmul_rn(ay, sd);
+          // performFFTScaling then performDensityCompensation
+          // (std_gpuNUFFT_kernels.cu:114-140, 220-242)
+          float ax = __fmul_rn(acc[c].x, scale);
+          float ay = __fmul_rn(acc[c].y, scale);
+          if (dens)
+          {
+            ax = __fmul_rn(ax, sd);
+            ay = __fmul_rn(ay, sd);
+          }
+          out[(size_t)cc * M + j] = make_float2(ax, ay);
         }
-        out[(size_t)(c0 + c) * M + j] = make_float2(ax, ay);
       }
     }
-  }
+  };
+  constexpr int P8 = CG >= 8 * MINC ? 8 : 1, P4 = CG >= 4 * MINC ? 4 : 1,
+                P2 = CG >= 2 * MINC ? 2 : 1;
+  if (P8 > 1 && n_samples <= kThreads / 8)
+    run(std::integral_constant<int, P8>());
+  else if (P4 > 1 && n_samples <= kThreads / 4)
+    run(std::integral_constant<int, P4>());
+  else if (P2 > 1 && n_samples <= kThreads / 2)
+    run(std::integral_constant<int, P2>());
+  else
+    run(std::integral_constant<int, 1>());
 }
 
 // The same interpolation with every coil group of an item in one block (3-D
@@ -1246,8 +1274,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
                          const float *__restrict__ dens,
                          const float2 *__restrict__ grid, Geo g,
                          const float *__restrict__ lut, uint32_t M, int C,
-                         int nbuf, float scale, float2 *__restrict__ out,
-                         tma::CopyWait cw)
+                         int nbuf, int x_shift, float scale,
+                         float2 *__restrict__ out, tma::CopyWait cw)
 {
   static_assert(CG % 2 == 0, "coil pairs");
   constexpr int NP = CG / 2;  // coil pairs per group
@@ -1268,6 +1296,7 @@ __global__ void __launch_bounds__(kThreads, MINB)
   int base[3];
   for (int a = 0; a < 3; ++a)
     base[a] = sa[a] * g.sw + (g.sw >> 1) - g.offset;
+  base[0] += x_shift;    // as stored
   constexpr int dx = 0;  // the box starts at the sector's own x
   bool inside = true;
   for (int a = 0; a < 3; ++a)
@@ -2131,6 +2160,12 @@ bool forward_pairs(const Geo &g, int tile_coils)
   return 2 * tile + 64 <= 74 * 1024;
 }
 
+int pair_x_shift(const Geo &g)
+{
+  const int first = (g.sw >> 1) - g.offset;  // first tile cell of sector 0
+  return g.sw % 8 == 0 ? (((-first) % 8) + 8) % 8 : 0;
+}
+
 // One block per work item: the bank group (16-byte unit mod 8) of each
 // sample's first footprint cell in the coil-pair tile, then the samples
 // dealt round-robin over the eight groups: position = the samples of lower
@@ -2243,7 +2278,7 @@ bool launch_forward_interp_tma(const FwdItem *items, int n_items,
         k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
     k<<<(unsigned)n_items, kThreads, smem2, s>>>(
         tm, items, lane_order, traj_sorted, idx, dens_sorted, grid, g, lut, M,
-        C, nbuf, scale, out, cw);
+        C, nbuf, pair_x_shift(g), scale, out, cw);
     GN_LAUNCH_CHECK("forward interpolation (coil-pair tiles, all groups)");
     return true;
   }
@@ -2309,6 +2344,8 @@ bool launch_forward_interp_tma(const FwdItem *items, int n_items,
 #define GN_TMA_KS(D, CGV)                                                      \
   if (ks == 4)                                                                 \
     GN_TMA(D, CGV, 4)                                                          \
+  else if (g.kw + 1 <= 6)                                                      \
+    GN_TMA(D, CGV, 6)                                                          \
   else                                                                         \
     GN_TMA(D, CGV, 8)
   if (g.dim == 3)

@@ -125,6 +125,12 @@ void build_forward_lane_order(const FwdItem *items, int n_items,
 // reads it).
 bool forward_pairs(const Geo &g, int tile_coils);
 
+// On that grid cell x is stored at x + pair_x_shift(g) mod G, so that the
+// rows of a sector's tile start on 128-byte lines (eight cells of a pair)
+// where the sector width is a multiple of eight: a row of ten cells then
+// lies in two lines instead of three.
+int pair_x_shift(const Geo &g);
+
 // --------------------------------------------------------------------------
 // Batches of independent operators: every stage of all instances in one
 // launch.  Each stage is a list of work units (instance, unit) with the

@@ -426,6 +426,13 @@ bool tile_rule(const gnufft_plan &p, uint32_t C)
   return C > 8 && work >= 6e6;
 }
 
+// The x shift of the column ranges: every separable forward of the plan
+// writes the same grid layout.
+int range_shift(const gnufft_plan &p)
+{
+  return forward_pairs(p.g, p.fwd_tile_coils) ? pair_x_shift(p.g) : 0;
+}
+
 void finish_tables(gnufft_plan &p)
 {
   // interpolation matrix (adjoint) and forward work items
@@ -453,8 +460,8 @@ void finish_tables(gnufft_plan &p)
     build_tile_tables(p.traj_sorted.as<float>(), p.sec_sorted.as<uint32_t>(),
                       p.M, p.g, p.lut.as<float>(), p.tiles, work, p.stream);
   if ((p.pruned || p.general) && p.dim == 3)
-    build_column_ranges(p.w_rows.as<uint32_t>(), p.g, p.zrange, p.ztiles,
-                        p.n_ztiles, p.stream);
+    build_column_ranges(p.w_rows.as<uint32_t>(), p.g, range_shift(p), p.zrange,
+                        p.ztiles, p.n_ztiles, p.stream);
   processing_order(p.sdc_h, p.order_h);
   upload(p.deapo, p.deapo_h.data(), p.deapo_h.size(), p.stream);
   GN_CUDA(cudaStreamSynchronize(p.stream));
@@ -690,6 +697,50 @@ size_t xrows_elems(const Geo &g, uint32_t C)
   return (size_t)C * g.G[2] * g.G[1] * g.N[0];
 }
 
+// Complex elements that one call with C coils needs of each scratch buffer.
+struct ScratchNeeds
+{
+  size_t ks = 0, grid = 0, fft_a = 0, fft_b = 0;
+  bool cufft = false;  // the call runs cuFFT (its plan holds a work area)
+  void merge(const ScratchNeeds &o)
+  {
+    ks = std::max(ks, o.ks);
+    grid = std::max(grid, o.grid);
+    fft_a = std::max(fft_a, o.fft_a);
+    fft_b = std::max(fft_b, o.fft_b);
+    cufft = cufft || o.cufft;
+  }
+  size_t bytes() const
+  {
+    return (ks + grid + fft_a + fft_b) * sizeof(float2);
+  }
+};
+
+ScratchNeeds adjoint_needs(const gnufft_plan &p, uint32_t C)
+{
+  const Geo &g = p.g;
+  const size_t cg = (size_t)spmm_coil_group((int)C);
+  ScratchNeeds n;
+  n.ks = (size_t)p.M * ((C + cg - 1) / cg * cg);
+  const bool tiled = tile_path(p, C);
+  n.cufft = !tiled && !p.pruned;
+  n.grid = (size_t)(tiled ? tile_grid_pitch((int)C) : (int)C) *
+           (size_t)g.grid_count;
+  if (!n.cufft)
+  {
+    n.fft_a = pruned_scratch_a(g, (int)C);
+    n.fft_b = std::max(pruned_scratch_b(g, (int)C),
+                       pruned_scratch_xfirst(g, (int)C));
+  }
+  if (tiled)
+  {
+    n.fft_a = std::max(n.fft_a, tile_partial_elems(p.tiles, g, (int)C));
+    size_t &rows = g.dim == 3 ? n.fft_b : n.fft_a;
+    rows = std::max(rows, xrows_elems(g, C));
+  }
+  return n;
+}
+
 // All coils of the call in one pass.
 void adjoint_batched(gnufft_plan &p, const float2 *k, float2 *img, uint32_t C,
                      int stage, cudaStream_t s, const float2 *sens,
@@ -723,23 +774,25 @@ void adjoint_batched(gnufft_plan &p, const float2 *k, float2 *img, uint32_t C,
      // transform to coil-major rows, then y and z
     check_copy_err(p);
     ensure_pruned(p, C, s);
-    p.fft_b.ensure(xrows_elems(g, C) * sizeof(float2));
-    // the partial columns live in the buffer of the coil-group sums, which
-    // come later
-    p.fft_a.ensure(tile_partial_elems(p.tiles, g, (int)C) * sizeof(float2));
+    // the partial columns are added up before the rows (2-D) or the
+    // coil-group sums (3-D) take their buffer
+    const ScratchNeeds need = adjoint_needs(p, C);
+    p.fft_a.ensure(need.fft_a * sizeof(float2));
+    p.fft_b.ensure(need.fft_b * sizeof(float2));
+    float2 *rows = g.dim == 3 ? p.fft_b.as<float2>() : p.fft_a.as<float2>();
     p.launches += launch_tile_spread(p.tiles, p.ks.as<float2>(), CP, g,
                                      (int)C, grid, p.fft_a.as<float2>(), s);
     p.mark(3, s);
     p.mark(4, s);
-    launch_tile_xpass(p.tiles, grid, g, (int)C, p.roots[0].as<float2>(),
-                      p.fft_b.as<float2>(), copy_wait(p), s);
+    launch_tile_xpass(p.tiles, grid, g, (int)C, p.roots[0].as<float2>(), rows,
+                      copy_wait(p), s);
     // the spread's grid is free once its rows are transformed: it takes the
-    // y pass's output
+    // y pass's output (3-D) or the coil-group sums (2-D)
     launch_pruned_adjoint_xfirst(
-        p.fft_b.as<float2>(), p.deapo.as<float>(),
+        rows, p.deapo.as<float>(),
         stage == GNUFFT_DEAPODIZATION ? sens : nullptr, g, (int)C,
         stage == GNUFFT_FFT ? 1 : 2, accumulate, root_ptrs(p).data(), grid,
-        p.fft_a.as<float2>(), img, s, copy_wait(p));
+        g.dim == 3 ? p.fft_a.as<float2>() : grid, img, s, copy_wait(p));
     p.launches += g.dim;
     p.mark(5, s);
     p.mark(6, s);
@@ -840,7 +893,8 @@ void forward_batched(gnufft_plan &p, const float2 *img, float2 *k, uint32_t C,
                           root_ptrs(p).data(), p.fft_a.as<float2>(),
                           p.fft_b.as<float2>(), grid, s,
                           p.zrange.as<uint2>(), copy_wait(p), paired,
-                          p.ztiles.as<uint32_t>(), p.n_ztiles, kColTile);
+                          p.ztiles.as<uint32_t>(), p.n_ztiles, kColTile,
+                          paired ? pair_x_shift(g) : 0);
     p.launches += g.dim;
     p.mark(5, s);
     p.mark(2, s);
@@ -931,25 +985,6 @@ void traj_grad(gnufft_plan &p, const float2 *img, const float2 *u, uint32_t C,
   p.launches += 3;
 }
 
-// Complex elements that one call with C coils needs of each scratch buffer.
-struct ScratchNeeds
-{
-  size_t ks = 0, grid = 0, fft_a = 0, fft_b = 0;
-  bool cufft = false;  // the call runs cuFFT (its plan holds a work area)
-  void merge(const ScratchNeeds &o)
-  {
-    ks = std::max(ks, o.ks);
-    grid = std::max(grid, o.grid);
-    fft_a = std::max(fft_a, o.fft_a);
-    fft_b = std::max(fft_b, o.fft_b);
-    cufft = cufft || o.cufft;
-  }
-  size_t bytes() const
-  {
-    return (ks + grid + fft_a + fft_b) * sizeof(float2);
-  }
-};
-
 ScratchNeeds forward_needs(const gnufft_plan &p, uint32_t C)
 {
   ScratchNeeds n;
@@ -961,30 +996,6 @@ ScratchNeeds forward_needs(const gnufft_plan &p, uint32_t C)
     n.fft_a = pruned_scratch_a(p.g, (int)C);
     n.fft_b = std::max(pruned_scratch_b(p.g, (int)C),
                        pruned_scratch_xfirst(p.g, (int)C));
-  }
-  return n;
-}
-
-ScratchNeeds adjoint_needs(const gnufft_plan &p, uint32_t C)
-{
-  const Geo &g = p.g;
-  const size_t cg = (size_t)spmm_coil_group((int)C);
-  ScratchNeeds n;
-  n.ks = (size_t)p.M * ((C + cg - 1) / cg * cg);
-  const bool tiled = tile_path(p, C);
-  n.cufft = !tiled && !p.pruned;
-  n.grid = (size_t)(tiled ? tile_grid_pitch((int)C) : (int)C) *
-           (size_t)g.grid_count;
-  if (!n.cufft)
-  {
-    n.fft_a = pruned_scratch_a(g, (int)C);
-    n.fft_b = std::max(pruned_scratch_b(g, (int)C),
-                       pruned_scratch_xfirst(g, (int)C));
-  }
-  if (tiled)
-  {
-    n.fft_b = std::max(n.fft_b, xrows_elems(g, C));
-    n.fft_a = std::max(n.fft_a, tile_partial_elems(p.tiles, g, (int)C));
   }
   return n;
 }
