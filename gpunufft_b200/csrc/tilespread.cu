@@ -5,7 +5,7 @@
 // issues about 70 instructions, 24 of them paired multiply-adds; a column is
 // written once.  3-D 128^3, 32 coils, 2.1 M samples on a B200: 0.92 ms for
 // the spread (3.4 records a sample) + 0.07 ms for the columns of several
-// chunks + 0.93 ms for the x transform (4.4 GB), against 2.87 ms for the CSR
+// chunks + 0.84 ms for the x transform (4.4 GB), against 2.87 ms for the CSR
 // product with the x transform fused, whose 27 gathers a sample wait on one
 // another.  Tiles of 4 x 4 x 4 cells, every row of a tile predicated per
 // record, took 1.54 ms (118 instructions a record, 12 warps an SM); 4 x 4 x
@@ -799,18 +799,22 @@ int reduce_tiles(const TileTables &t, const float2 *partial, int HP, int C,
 // stage 2 runs with lanes over k1, which then meet different banks and write
 // consecutive x.  Bound by instruction issue (3-D 128^3, 32 coils: 1.18 ms
 // with all outputs' addresses and range tests, 0.93 ms with HALF, which also
-// drops the last butterflies' unused outputs; 4.4 GB at the HBM copy rate
-// take 0.66 ms).
+// drops the last butterflies' unused outputs, 0.84 ms with two coils per
+// thread; 4.4 GB at the HBM copy rate take 0.66 ms).
 template <int L, int CB, int TX> struct XPass
 {
   using S = fftcore::Shape<L>;
-  static constexpr int NT = CB * S::T < 32 ? 32 : CB * S::T;
+  // two coils per thread (16-byte shared accesses, one address and twiddle
+  // for both): 3-D 128^3, 32 coils 0.90 -> 0.84 ms; 128-point rows of 8 coils
+  // (64^3) 40 -> 42 us, and 512-point rows would not fit the registers
+  static constexpr int CPT = L == 256 && CB == 16 ? 2 : 1;
+  static constexpr int NT = CB / CPT * S::T < 32 ? 32 : CB / CPT * S::T;
   // two row buffers; one where two do not fit
   static constexpr int NBUF = (size_t)L * CB * 16 > 200 * 1024 ? 1 : 2;
   static constexpr size_t smem =
       ((size_t)NBUF * L * CB + L) * sizeof(float2) + 2 * 8 + 16;
   static constexpr int OW = (L / TX + 31) / 32;  // occupancy words per row
-  static constexpr int WANT = L >= 512 ? 512 : 768;  // threads per SM
+  static constexpr int WANT = L >= 512 ? 512 : 768 / CPT;  // threads per SM
   static constexpr int MINB = WANT / NT > 6 ? 6 : (NT > WANT ? 1 : WANT / NT);
 };
 
@@ -928,56 +932,89 @@ __global__ void __launch_bounds__(XPass<L, CB, TX>::NT,
       }
       return;
     }
+    constexpr int CPT = XPass<L, CB, TX>::CPT, CV = CB / CPT;
+    auto occupied = [&](int j, int r) {
+      // FFT input n holds cell (n + L / 2) mod L, of the same residue class
+      // mod R2: input r + R2 j is cell r + R2 jj.  With R2 a multiple of TX
+      // (or TX of R2) the word and most of the shift are constants.
+      const int jj = (j + S::R1 / 2) % S::R1;
+      const int tb = S::R2 % TX == 0 ? S::R2 / TX * jj : 0;
+      const int ti = S::R2 % TX == 0 ? r / TX : (r + S::R2 * jj) / TX;
+      return ((cur.w[(S::R2 % TX == 0 ? tb : S::R2 * jj / TX) >> 5] >>
+               (ti & 31)) &
+              (1u << (tb & 31))) != 0u;
+    };
     {
-      const int c = threadIdx.x % CB, r = threadIdx.x / CB;
-      float2 a[S::R1];
+      const int c = threadIdx.x % CV, r = threadIdx.x / CV;
+      float2 a[CPT][S::R1];
       if (r < S::R2)
       {
-        // FFT input n holds cell (n + L / 2) mod L, of the same residue
-        // class mod R2
 #pragma unroll
         for (int j = 0; j < S::R1; ++j)
         {
           const int jj = (j + S::R1 / 2) % S::R1;
-          // tile of cell r + R2 jj; with R2 a multiple of TX (or TX of R2)
-          // the word and most of the shift are constants
-          const int tb = S::R2 % TX == 0 ? S::R2 / TX * jj : 0;
-          const int ti = S::R2 % TX == 0 ? r / TX : (r + S::R2 * jj) / TX;
-          const bool on =
-              (cur.w[(S::R2 % TX == 0 ? tb : S::R2 * jj / TX) >> 5] >>
-               (ti & 31)) &
-              (1u << (tb & 31));
-          a[j] = on ? buf[(r + S::R2 * jj) * CB + c] : make_float2(0.f, 0.f);
+          const bool on = occupied(j, r);
+          if constexpr (CPT == 2)
+          {
+            const float4 q =
+                on ? reinterpret_cast<const float4 *>(
+                         buf)[(r + S::R2 * jj) * CV + c]
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+            a[0][j] = make_float2(q.x, q.y);
+            a[CPT - 1][j] = make_float2(q.z, q.w);
+          }
+          else
+            a[0][j] = on ? buf[(r + S::R2 * jj) * CB + c]
+                         : make_float2(0.f, 0.f);
         }
       }
       __syncwarp();
       if (r < S::R2)
       {
-        fftcore::reg_fft<S::R1, fftcore::Rm<L>::V, true>(a, w);
+#pragma unroll
+        for (int v = 0; v < CPT; ++v)
+          fftcore::reg_fft<S::R1, fftcore::Rm<L>::V, true>(a[v], w);
 #pragma unroll
         for (int k1 = 0; k1 < S::R1; ++k1)
         {
-          float2 v = a[k1];
           if (k1 != 0)
           {
             float2 t = tw[r * k1];
             t.y = -t.y;
-            v = cmul(v, t);
+#pragma unroll
+            for (int v = 0; v < CPT; ++v)
+              a[v][k1] = cmul(a[v][k1], t);
           }
-          buf[(r + S::R2 * k1) * CB + (c ^ (k1 & (CB - 1)))] = v;
+          const int at = (r + S::R2 * k1) * CV + (c ^ (k1 & (CV - 1)));
+          if constexpr (CPT == 2)
+            reinterpret_cast<float4 *>(buf)[at] =
+                make_float4(a[0][k1].x, a[0][k1].y, a[CPT - 1][k1].x,
+                            a[CPT - 1][k1].y);
+          else
+            buf[at] = a[0][k1];
         }
       }
     }
     __syncthreads();
     const int k1 = threadIdx.x % S::T, cl = threadIdx.x / S::T;
-    const int c = c_first + (int)gi * CB + cl;
-    float2 bb[S::R2];
-    const bool live = k1 < S::R1 && cl < CB && c < C;
+    const int c = c_first + (int)gi * CB + cl * CPT;
+    float2 bb[CPT][S::R2];
+    const bool live = k1 < S::R1 && cl < CV && c < C;
     if (live)
     {
 #pragma unroll
       for (int r = 0; r < S::R2; ++r)
-        bb[r] = buf[(r + S::R2 * k1) * CB + (cl ^ (k1 & (CB - 1)))];
+      {
+        const int at = (r + S::R2 * k1) * CV + (cl ^ (k1 & (CV - 1)));
+        if constexpr (CPT == 2)
+        {
+          const float4 q = reinterpret_cast<const float4 *>(buf)[at];
+          bb[0][r] = make_float2(q.x, q.y);
+          bb[CPT - 1][r] = make_float2(q.z, q.w);
+        }
+        else
+          bb[0][r] = buf[at];
+      }
     }
     tma::fence_proxy_async();  // the in-place writes before the refill
     __syncthreads();           // buffer b is free
@@ -985,27 +1022,34 @@ __global__ void __launch_bounds__(XPass<L, CB, TX>::NT,
       issue(u + NBUF * stride, b, NBUF == 2 ? nn : nxt);
     if (live)
     {
-      fftcore::reg_fft<S::R2, fftcore::Rm<L>::V, true>(bb, w);
       float2 *o = out + (long long)c * plane +
                   ((long long)z * g.G[1] + y) * Nx;
-      if constexpr (HALF)
-      {  // N = G / 2: the outputs k < L / 4 and k >= 3 L / 4, constant steps
-        o += k1 + L / 4;
 #pragma unroll
-        for (int k2 = 0; k2 < S::R2 / 4; ++k2)
-        {
-          o[S::R1 * k2] = bb[k2];
-          o[S::R1 * (k2 - S::R2 / 4)] = bb[k2 + 3 * S::R2 / 4];
-        }
-      }
-      else
+      for (int v = 0; v < CPT; ++v)
       {
+        if (v > 0 && c + v >= C)
+          break;
+        fftcore::reg_fft<S::R2, fftcore::Rm<L>::V, true>(bb[v], w);
+        float2 *ov = o + v * plane;
+        if constexpr (HALF)
+        {  // N = G / 2: the outputs k < L / 4 and k >= 3 L / 4, constant steps
+          ov += k1 + L / 4;
 #pragma unroll
-        for (int k2 = 0; k2 < S::R2; ++k2)
+          for (int k2 = 0; k2 < S::R2 / 4; ++k2)
+          {
+            ov[S::R1 * k2] = bb[v][k2];
+            ov[S::R1 * (k2 - S::R2 / 4)] = bb[v][k2 + 3 * S::R2 / 4];
+          }
+        }
+        else
         {
-          const int x = (k1 + S::R1 * k2 + add) & (L - 1);
-          if (x < Nx)
-            o[x] = bb[k2];
+#pragma unroll
+          for (int k2 = 0; k2 < S::R2; ++k2)
+          {
+            const int x = (k1 + S::R1 * k2 + add) & (L - 1);
+            if (x < Nx)
+              ov[x] = bb[v][k2];
+          }
         }
       }
     }
