@@ -25,6 +25,7 @@ CONVOLUTION, FFT, DEAPODIZATION, DENSITY_ESTIMATION = 0, 1, 2, 3
 FLAG_REFERENCE_ORDER = 0x1
 FLAG_PLAIN = 0x2
 FLAG_CUFFT = 0x4
+CG_WORK_BYTES = 8192  # GNUFFT_CG_WORK_BYTES
 # GNUFFT_NOALLOC_SCRATCH_BYTES: staging area of the no-allocation adjoint
 NOALLOC_SCRATCH_BYTES = 16 << 20
 
@@ -42,7 +43,8 @@ EXPORTED = (
     "gnufft_plan_create", "gnufft_plan_load", "gnufft_plan_destroy",
     "gnufft_plan_get_info", "gnufft_export_tables", "gnufft_set_sens",
     "gnufft_adjoint_host", "gnufft_adjoint_device", "gnufft_forward_host",
-    "gnufft_forward_device", "gnufft_set_timing", "gnufft_get_stage_times",
+    "gnufft_forward_device", "gnufft_cg_begin", "gnufft_cg_step",
+    "gnufft_set_timing", "gnufft_get_stage_times",
     "gnufft_last_error", "gnufft_status_string", "gnufft_version",
     "gnufft_adjoint_convolution_noalloc",
     "gnufft_traj_grad_device", "gnufft_set_sens_device",
@@ -147,6 +149,10 @@ def lib() -> ctypes.CDLL:
         f.argtypes = [_P, _P, _P, _U, _I, _P]
     L.gnufft_adjoint_convolution_noalloc.restype = st
     L.gnufft_adjoint_convolution_noalloc.argtypes = [_P, _P, _P, _U, _P]
+    L.gnufft_cg_begin.restype = st
+    L.gnufft_cg_begin.argtypes = [_P, _P, ctypes.c_uint64, _P, _P]
+    L.gnufft_cg_step.restype = st
+    L.gnufft_cg_step.argtypes = [_P, _P, _P, _P, _P, ctypes.c_uint64, _P, _P]
     L.gnufft_traj_grad_device.restype = st
     L.gnufft_traj_grad_device.argtypes = [_P, _P, _P, _U, _P, _P]
     L.gnufft_set_timing.restype = st

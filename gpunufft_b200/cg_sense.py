@@ -10,23 +10,48 @@ and ``maxit`` plain conjugate-gradient iterations from x = 0 (the upstream
 loop ignores ``tol``; so does this one unless ``tol`` is given).  Pruessmann
 et al., MRM 46:638-651 (2001).
 
-All vector arithmetic runs in torch on the current CUDA stream; the operator
-applications go through the C ABI on the same stream, so a whole solve is
-stream-ordered and needs no host synchronisation until the caller reads the
-result.
+The operator applications and the vector updates (``gnufft_cg_step``: three
+launches per iteration, scalars on the device) go through the C ABI on the
+current CUDA stream, so a whole solve is stream-ordered and needs no host
+synchronisation until the caller reads the result.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Callable, Optional
 
 import torch
 
+from . import _capi as C
 from .operator import Plan
 
 
-def _dot(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
-    """<a, b> = sum(conj(a) * b) as a 0-d complex tensor on the device."""
-    return torch.vdot(a.reshape(-1), b.reshape(-1))
+class CgVectors:
+    """The vectors of one solve of M x = rhs on the current CUDA stream:
+    ``x``, the residual ``r`` (takes ``rhs`` over) and the direction ``p``,
+    updated in place by ``step``; ``rr`` is ||r||^2 on the device."""
+
+    def __init__(self, plan: Plan, rhs: torch.Tensor):
+        self.plan = plan
+        self.x = torch.zeros_like(rhs)
+        self.r = rhs
+        self.p = rhs.clone()
+        self.work = torch.empty(C.CG_WORK_BYTES // 4, dtype=torch.float32,
+                                device=rhs.device)
+        C.check(C.lib().gnufft_cg_begin(plan._h, rhs.data_ptr(), rhs.numel(),
+                                        self.work.data_ptr(), self._stream()))
+        self.rr = self.work[0]
+
+    def _stream(self) -> ctypes.c_void_p:
+        return ctypes.c_void_p(
+            torch.cuda.current_stream(self.r.device).cuda_stream)
+
+    def step(self, ap: torch.Tensor) -> None:
+        """One iteration, with ``ap`` = M p."""
+        C.check(C.lib().gnufft_cg_step(
+            self.plan._h, self.x.data_ptr(), self.r.data_ptr(),
+            self.p.data_ptr(), ap.data_ptr(), self.r.numel(),
+            self.work.data_ptr(), self._stream()))
 
 
 def cg_sense(plan: Plan, kspace: torch.Tensor, maxit: int = 10,
@@ -57,22 +82,12 @@ def cg_sense(plan: Plan, kspace: torch.Tensor, maxit: int = 10,
             out = out + alpha * v
         return out
 
-    x = torch.zeros_like(rhs)
-    r = rhs.clone()
-    p = r.clone()
-    rr = _dot(r, r).real
-    stop = None if tol is None else (tol ** 2) * rr
+    v = CgVectors(plan, rhs)
+    stop = None if tol is None else (tol ** 2) * v.rr
     for it in range(maxit):
-        ap = apply_m(p)
-        a = rr / _dot(p, ap)
-        x = x + a * p
-        r = r - a * ap
-        rr_new = _dot(r, r).real
-        b = rr_new / rr
-        rr = rr_new
-        p = r + b * p
+        v.step(apply_m(v.p))
         if callback is not None:
-            callback(it, x)
-        if stop is not None and bool(rr <= stop):
+            callback(it, v.x.clone())  # x is updated in place
+        if stop is not None and bool(v.rr <= stop):
             break
-    return x
+    return v.x

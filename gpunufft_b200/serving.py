@@ -29,7 +29,7 @@ import numpy as np
 import torch
 
 from . import _capi as C
-from .cg_sense import _dot
+from .cg_sense import CgVectors
 from .operator import Plan
 
 
@@ -250,24 +250,17 @@ class _Active:
             self.y = torch.as_tensor(req.kspace).to(dev, non_blocking=True)
             self.maps = torch.as_tensor(req.sens).to(dev, non_blocking=True)
             plan.set_sens(self.maps)
-            rhs = plan.adjoint(self.y)
-            self.x = torch.zeros_like(rhs)
-            self.r = rhs
-            self.p = rhs.clone()
-            self.rr = _dot(self.r, self.r).real
+            self.cg = CgVectors(plan, plan.adjoint(self.y))
+            self.x = self.cg.x
 
     def _iteration(self) -> None:
         """One CG iteration (matlab/demo/utils/cg_sense_2d.m:76-100) with
-        in-place updates of x, r, p and rr."""
-        ap = self.plan.adjoint(self.plan.forward(self.p))
+        in-place updates of the solve's vectors."""
+        p = self.cg.p
+        ap = self.plan.adjoint(self.plan.forward(p))
         if self.req.alpha:
-            ap = ap + self.req.alpha * self.p
-        a = self.rr / _dot(self.p, ap)
-        self.x.add_(a * self.p)
-        self.r.sub_(a * ap)
-        rr_new = _dot(self.r, self.r).real
-        self.p.mul_(rr_new / self.rr).add_(self.r)
-        self.rr.copy_(rr_new)
+            ap = ap + self.req.alpha * p
+        self.cg.step(ap)
 
     def step(self) -> None:
         """Enqueue one CG iteration on this request's stream."""

@@ -263,6 +263,24 @@ GNUFFT_API gnufft_status gnufft_traj_grad_device(gnufft_plan *plan, const void *
                                       uint32_t n_coils, float *grad_traj,
                                       void *stream);
 
+/* Vector updates of a conjugate-gradient solve of M x = b (no upstream
+ * counterpart; used by the CG-SENSE solver), complex64 vectors of n elements
+ * on the plan's device.  `work`: GNUFFT_CG_WORK_BYTES of device memory
+ * (16-byte aligned) that holds the scalars of one solve; its first float is
+ * ||residual||^2.  gnufft_cg_begin starts a solve.  gnufft_cg_step makes one
+ * iteration with image = M direction:
+ *   a = ||r||^2 / <direction, image>, x += a direction, r -= a image,
+ *   direction = r + (||r_new||^2 / ||r||^2) direction.
+ * Both are ordered on `stream`; the sums have a fixed order. */
+#define GNUFFT_CG_WORK_BYTES 8192
+GNUFFT_API gnufft_status gnufft_cg_begin(const gnufft_plan *plan,
+                                         const void *residual, uint64_t n,
+                                         void *work, void *stream);
+GNUFFT_API gnufft_status gnufft_cg_step(const gnufft_plan *plan, void *x,
+                                        void *residual, void *direction,
+                                        const void *image, uint64_t n,
+                                        void *work, void *stream);
+
 /* Device time (ms) of the stages of the last call on this plan, measured
  * with CUDA events when timing is enabled (gnufft_set_timing). */
 typedef struct gnufft_stage_times {

@@ -86,3 +86,55 @@ def test_cg_sense_reduces_the_residual_and_beats_the_adjoint():
     err_adj = float(torch.linalg.vector_norm(s * xa - x_true) /
                     torch.linalg.vector_norm(x_true))
     assert err_cg < err_adj, (err_cg, err_adj)
+
+
+@pytest.mark.parametrize("n", [1, 255, 1024, 1025, 70_001, 444 * 1024 + 3])
+def test_cg_vector_updates(n):
+    """gnufft_cg_begin / gnufft_cg_step against float64, from one element to
+    more elements than the blocks take four at a time; repeated calls give
+    the same bits."""
+    import ctypes
+
+    import torch
+
+    import gpunufft_b200 as G
+    from gpunufft_b200 import _capi as C
+    plan = G.Plan(np.zeros((2, 4), np.float32), (16, 16))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+
+    def vec():
+        return torch.randn(n, generator=g, device="cuda",
+                           dtype=torch.complex64)
+    x0, r0, p0, q = vec(), vec(), vec(), vec()
+    q = p0 + 0.25 * q  # <p, q> away from zero
+    outs = []
+    for _ in range(2):
+        x, r, p = x0.clone(), r0.clone(), p0.clone()
+        work = torch.empty(C.CG_WORK_BYTES // 4, device="cuda")
+        s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        C.check(C.lib().gnufft_cg_begin(plan._h, r.data_ptr(), n,
+                                        work.data_ptr(), s))
+        rr0 = float(work[0])
+        C.check(C.lib().gnufft_cg_step(plan._h, x.data_ptr(), r.data_ptr(),
+                                       p.data_ptr(), q.data_ptr(), n,
+                                       work.data_ptr(), s))
+        outs.append((x, r, p, work[:1].clone()))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    d = [t.to(torch.complex128) for t in (x0, r0, p0, q)]
+    rr = torch.vdot(d[1], d[1]).real
+    a = rr / torch.vdot(d[2], d[3])
+    want_x, want_r = d[0] + a * d[2], d[1] - a * d[3]
+    rn = torch.vdot(want_r, want_r).real
+    want_p = want_r + (rn / rr) * d[2]
+    # sums in double, vectors in single: a few roundings of 6e-8 of the terms
+    norm = torch.linalg.vector_norm
+    assert abs(rr0 - float(rr)) < 2e-7 * float(rr)
+    terms = (norm(d[0]) + norm(a * d[2]), norm(d[1]) + norm(a * d[3]),
+             norm(want_r) + norm((rn / rr) * d[2]) + norm(d[1]) +
+             norm(a * d[3]))
+    for got, want, t in zip(outs[0], (want_x, want_r, want_p), terms):
+        assert float(norm(got - want) / t) < 1e-6
+    assert abs(float(outs[0][3][0]) - float(rn)) < 1e-6 * float(terms[1]) ** 2
+    plan.close()
