@@ -29,6 +29,7 @@ struct gnufft_batch
   DeviceBuffer inst_d, arena, counters;
   uint32_t total[kBatchStages] = {};
   size_t interp_smem = 0;
+  int slots = 4;  // most footprint slots of an instance
   BatchIo io{};  // per-call data pointers (kernel parameter)
   // the transforms run on side streams forked from the caller's stream;
   // instances that share a cuFFT plan (frames of one plan) share a side
@@ -159,6 +160,7 @@ gnufft_status gnufft_batch_create(gnufft_plan *const *plans,
         throw Error(kNotSupported,
                     who + "forward tile exceeds shared memory");
       b->interp_smem = std::max(b->interp_smem, smem);
+      b->slots = std::max(b->slots, bi.slots);
       b->fft[i] = t.fft;
       grid_off[i] = bytes;
       bytes += align256((size_t)C * t.g.grid_count * sizeof(float2));
@@ -238,13 +240,14 @@ gnufft_status gnufft_batch_forward(gnufft_batch *b, const void *const *images,
     const BatchInst *inst = b->inst_d.as<BatchInst>();
     GN_CUDA(cudaMemsetAsync(cnt, 0, kBatchStages * sizeof(unsigned), s));
     launch_batch_stage(kBatchPrepare, inst, (int)b->n, b->total[kBatchPrepare],
-                       &b->io, cnt + kBatchPrepare, 0, s);
+                       &b->io, cnt + kBatchPrepare, 0, b->slots, s);
     run_ffts(*b, CUFFT_FORWARD, s);
     launch_batch_stage(kBatchInterp, inst, (int)b->n, b->total[kBatchInterp],
-                       &b->io, cnt + kBatchInterp, b->interp_smem, s);
+                       &b->io, cnt + kBatchInterp, b->interp_smem, b->slots,
+                       s);
     launch_batch_stage(kBatchInterp3, inst, (int)b->n,
                        b->total[kBatchInterp3], &b->io, cnt + kBatchInterp3,
-                       b->interp_smem, s);
+                       b->interp_smem, b->slots, s);
   });
 }
 
@@ -268,12 +271,12 @@ gnufft_status gnufft_batch_adjoint(gnufft_batch *b, const void *const *kspace,
     const BatchInst *inst = b->inst_d.as<BatchInst>();
     GN_CUDA(cudaMemsetAsync(cnt, 0, kBatchStages * sizeof(unsigned), s));
     launch_batch_stage(kBatchGather, inst, (int)b->n, b->total[kBatchGather],
-                       &b->io, cnt + kBatchGather, 0, s);
+                       &b->io, cnt + kBatchGather, 0, b->slots, s);
     launch_batch_stage(kBatchSpread, inst, (int)b->n, b->total[kBatchSpread],
-                       &b->io, cnt + kBatchSpread, 0, s);
+                       &b->io, cnt + kBatchSpread, 0, b->slots, s);
     run_ffts(*b, CUFFT_INVERSE, s);
     launch_batch_stage(kBatchFinish, inst, (int)b->n, b->total[kBatchFinish],
-                       &b->io, cnt + kBatchFinish, 0, s);
+                       &b->io, cnt + kBatchFinish, 0, b->slots, s);
   });
 }
 

@@ -192,10 +192,11 @@ size_t batch_interp_smem(const BatchInst &b);
 // One launch of `stage` over the n instances (device array `inst`, units
 // `total`); `counter` (device, zero before the launch) hands out the units.
 // `io` carries the inputs / outputs of the stages that read or write the
-// caller's data.  Returns the number of blocks launched.
+// caller's data; `slots`: the most footprint slots of an instance.  Returns
+// the number of blocks launched.
 unsigned launch_batch_stage(int stage, const BatchInst *inst, int n,
                             uint32_t total, const BatchIo *io,
-                            unsigned *counter, size_t interp_smem,
+                            unsigned *counter, size_t interp_smem, int slots,
                             cudaStream_t s);
 
 }  // namespace gnufft
