@@ -475,8 +475,8 @@ __global__ void k_col_ranges(const uint32_t *__restrict__ row_off, int G0,
 }  // namespace
 
 void build_column_ranges(const uint32_t *row_off, const Geo &g, int x_shift,
-                         DeviceBuffer &range, DeviceBuffer &tiles,
-                         int &n_tiles, cudaStream_t s)
+                         DeviceBuffer &range, DeviceBuffer &yrange,
+                         DeviceBuffer &tiles, int &n_tiles, cudaStream_t s)
 {
   const size_t cols = (size_t)g.G[0] * g.G[1];
   range.reset(cols * sizeof(uint2));
@@ -489,6 +489,18 @@ void build_column_ranges(const uint32_t *row_off, const Geo &g, int x_shift,
   GN_CUDA(cudaMemcpyAsync(h.data(), range.get(), cols * sizeof(uint2),
                           cudaMemcpyDeviceToHost, s));
   GN_CUDA(cudaStreamSynchronize(s));
+  // per stored x the y rows that hold a range
+  std::vector<uint2> yr(g.G[0], make_uint2(0xFFFFFFFFu, 0u));
+  for (int y = 0; y < g.G[1]; ++y)
+    for (int x = 0; x < g.G[0]; ++x)
+      if (h[(size_t)y * g.G[0] + x].x <= h[(size_t)y * g.G[0] + x].y)
+      {
+        yr[x].x = std::min(yr[x].x, (uint32_t)y);
+        yr[x].y = (uint32_t)y;
+      }
+  yrange.reset(yr.size() * sizeof(uint2));
+  GN_CUDA(cudaMemcpyAsync(yrange.get(), yr.data(), yr.size() * sizeof(uint2),
+                          cudaMemcpyHostToDevice, s));
   // tiles of kColTile adjacent columns with at least one range
   std::vector<uint32_t> list;
   const size_t nt = (cols + kColTile - 1) / kColTile;

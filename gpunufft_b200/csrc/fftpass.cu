@@ -1599,7 +1599,8 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
                            const float *deapo, const Geo &g, int C,
                            const float2 *const roots[3], float2 *tmp_a,
                            float2 *tmp_b, float2 *grid, cudaStream_t s,
-                           const uint2 *zrange, tma::CopyWait cw,
+                           const uint2 *zrange, const uint2 *yrange,
+                           tma::CopyWait cw,
                            bool paired, const uint32_t *ztiles, int n_ztiles,
                            int ztile_cols, int x_shift)
 {
@@ -1642,7 +1643,7 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
               (long long)C * g.N[2],
               pos_mod((long long)g.shift_inv[1] - g.crop[1], g.G[1]), g.N[1],
               pos_mod(-(long long)g.shift_fwd[1], g.G[1]), g.G[1], roots[1],
-              s, nullptr, cw);
+              s, g.dim == 3 ? yrange : nullptr, cw);
   if (g.dim == 3)  // z: B -> grid
     cols<false>(g.G[2], tmp_b, grid, (long long)g.G[1] * g.G[0], g.N[2],
                 g.G[2], C,

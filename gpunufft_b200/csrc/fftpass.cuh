@@ -48,8 +48,8 @@ size_t pruned_scratch_b(const Geo &g, int C);
 // -> FORWARD fftshift -> grid [C][G] (so cell q of the shifted spectrum, the
 // one the interpolation reads, is stored at q).
 // roots[a]: the root table of axis a (length G[a]).
-// zrange (3-D, optional): per (y, x) column the z rows to write; the
-// others are left as they are (the interpolation never reads them).
+// zrange, yrange (3-D, optional): per (y, x) column the z rows to write, per
+// x the y rows of the y pass's output to write; the others are left as they are (the interpolation never reads them).
 // err (optional): the mapped error flag of the tensor-copy passes (set when
 // a tile copy does not complete within its bounded wait); without it the
 // passes load their tiles with plain loads.  paired (3-D, needs err and
@@ -64,6 +64,7 @@ void launch_pruned_forward(const float2 *image, const float2 *sens,
                            const float2 *const roots[3], float2 *tmp_a,
                            float2 *tmp_b, float2 *grid, cudaStream_t s,
                            const uint2 *zrange = nullptr,
+                           const uint2 *yrange = nullptr,
                            tma::CopyWait cw = tma::CopyWait(),
                            bool paired = false,
                            const uint32_t *ztiles = nullptr, int n_ztiles = 0,

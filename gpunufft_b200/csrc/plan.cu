@@ -98,6 +98,7 @@ struct gnufft_plan
   DeviceBuffer dlut;          // kernel derivative table (trajectory gradient)
   DeviceBuffer roots[3];      // DFT roots per axis (pruned transforms)
   DeviceBuffer zrange;        // per (y, x) column: z rows with weights
+  DeviceBuffer yrange;        // per x: y rows with a z range
   DeviceBuffer ztiles;        // column tiles holding a z range
   TileTables tiles;           // records of the tile spread (adjoint)
   int n_ztiles = 0;
@@ -153,7 +154,7 @@ struct gnufft_plan
                                   &stage_out,   &one_sens,    &fft_a,
                                   &fft_b,       &dlut,        &roots[0],
                                   &roots[1],    &roots[2],    &zrange,
-                                  &ztiles};
+                                  &yrange,      &ztiles};
     size_t s = tiles.bytes();
     for (auto *b : bufs)
       s += b->bytes();
@@ -461,7 +462,7 @@ void finish_tables(gnufft_plan &p)
                       p.M, p.g, p.lut.as<float>(), p.tiles, work, p.stream);
   if ((p.pruned || p.general) && p.dim == 3)
     build_column_ranges(p.w_rows.as<uint32_t>(), p.g, range_shift(p), p.zrange,
-                        p.ztiles, p.n_ztiles, p.stream);
+                        p.yrange, p.ztiles, p.n_ztiles, p.stream);
   processing_order(p.sdc_h, p.order_h);
   upload(p.deapo, p.deapo_h.data(), p.deapo_h.size(), p.stream);
   GN_CUDA(cudaStreamSynchronize(p.stream));
@@ -892,7 +893,8 @@ void forward_batched(gnufft_plan &p, const float2 *img, float2 *k, uint32_t C,
     launch_pruned_forward(img, sens, p.deapo.as<float>(), g, (int)C,
                           root_ptrs(p).data(), p.fft_a.as<float2>(),
                           p.fft_b.as<float2>(), grid, s,
-                          p.zrange.as<uint2>(), copy_wait(p), paired,
+                          p.zrange.as<uint2>(), p.yrange.as<uint2>(),
+                          copy_wait(p), paired,
                           p.ztiles.as<uint32_t>(), p.n_ztiles, kColTile,
                           paired ? pair_x_shift(g) : 0);
     p.launches += g.dim;

@@ -89,7 +89,7 @@ def plan_table_bytes(req: Request) -> int:
         b += 4 * M
     b += 16 * (M // 256 + int(np.prod([-(-g // req.sector_width)
                                        for g in grid])) + 1)
-    b += 8 * grid[0] * grid[1] + 4 * (grid[0] * grid[1] // 8 + 1)
+    b += 8 * grid[0] * (grid[1] + 1) + 4 * (grid[0] * grid[1] // 8 + 1)
     b += 4 * N + 4 * 4096 + 8 * Cn * N
     cells = req.kernel_width + 1
     planes = 4 if cells <= 4 else (6 if cells <= 6 else 8)
