@@ -1,7 +1,8 @@
 // Per-call kernels of the operator path (sm_100a).
 //
 // Adjoint: the sorted k-space is gathered coil-interleaved (one row of coil
-// values per sample), then spread as a sparse product with the plan's
+// values per sample), then spread by register columns (tilespread.cu) or,
+// for few coils and small work, here as a sparse product with the plan's
 // interpolation matrix: one block per grid row chunk and coil group streams
 // the chunk's nonzeros in equal shares per unit of lanes, keeps running
 // cell sums in registers and finishes cells cut by share boundaries in
