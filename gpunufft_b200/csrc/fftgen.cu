@@ -6,7 +6,7 @@
 // the way in and out.
 //
 // Bound by instruction issue and the latency of short blocks.  3-D 96^3 on
-// 192^3, 16 coils on a B200: forward x / y / z 0.15 / 0.18 / 0.33 ms where
+// 192^3, 16 coils on a B200: forward x / y / z 0.15 / 0.18 / 0.31 ms where
 // cuFFT and the padding pass took 1.30 ms over the whole zero-padded grid;
 // adjoint x / y / z with the coil sum 0.36 / 0.18 / 0.15 ms against 1.12 ms.
 #include "fftgen.cuh"
@@ -73,24 +73,47 @@ template <bool SWAP> __device__ __forceinline__ float2 part_swap(float2 v)
 // q = k0 R1 + k1 of the last stage reads rows q R2 + r and gives outputs
 // k0 + R0 (k1 + R1 k2): store(k0 + R0 k1, R0 R1, a).  A barrier precedes
 // each later stage.
-template <int PITCH, class Load, class Store>
+//
+// EARLY: ready() brings the roots to shared memory (and holds a barrier)
+// between a thread's first loads and its use of the roots, while the loads
+// are in flight.  Column passes only: 3-D 96^3 on 192^3, 16 coils on a
+// B200, the whole forward 0.97 -> 0.95 ms; in the x pass and the coil sum,
+// which keep more values across it, it spills (0.36 -> 0.38 ms, 0.15 ->
+// 0.19 ms).
+template <int PITCH, bool EARLY, class Ready, class Load, class Store>
 __device__ __forceinline__ void line_dft(const Factors &f, float2 *buf, int cl,
                                          int lt, bool on, const float2 *tw,
-                                         Load load, Store store)
+                                         Ready ready, Load load, Store store)
 {
   const int M = f.L / f.R[0];
-  if (on)
-    for (int r = lt; r < M; r += f.threads)
-      with_radix(f.R[0], [&](auto &a) {
-        constexpr int R = sizeof(a) / sizeof(a[0]);
-        load(r, M, a);
-        transform(a);
-        float2 *q = buf + r * PITCH + cl;
-        q[0] = a[0];
-        const int step = M * PITCH;
+  auto finish = [&](int r, auto &a) {
+    constexpr int R = sizeof(a) / sizeof(a[0]);
+    transform(a);
+    float2 *q = buf + r * PITCH + cl;
+    q[0] = a[0];
+    const int step = M * PITCH;
 #pragma unroll
-        for (int k = 1; k < R; ++k)
-          q[k * step] = cmul(a[k], tw[k * r]);
+    for (int k = 1; k < R; ++k)
+      q[k * step] = cmul(a[k], tw[k * r]);
+  };
+  int r0 = lt;
+  if (EARLY)
+  {
+    with_radix(f.R[0], [&](auto &a) {
+      const bool act = on && lt < M;
+      if (act)
+        load(lt, M, a);
+      ready();
+      if (act)
+        finish(lt, a);
+    });
+    r0 += f.threads;
+  }
+  if (on)
+    for (int r = r0; r < M; r += f.threads)
+      with_radix(f.R[0], [&](auto &a) {
+        load(r, M, a);
+        finish(r, a);
       });
   __syncthreads();
   if (f.R[1] > 1)
@@ -146,7 +169,6 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
 {
   extern __shared__ float2 sm[];
   float2 *tw = sm, *buf = sm + f.L;
-  fftcore::load_roots(tw, roots, f.L);
   const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
   long long plane, col;
   if (PAIRED)
@@ -170,14 +192,17 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
     lo = cr.x;
     span = min(cr.y + 1, span) - lo;
   }
-  __syncthreads();
   const float2 *sp = src + plane * src_rows * ncols + col;
   const long long psz = (long long)dst_rows * ncols;
   float2 *dp = PAIRED ? dst + ((plane >> 1) * psz + col) * 2 + (plane & 1)
                       : dst + plane * psz + col;
   const uint32_t is = (uint32_t)ncols, os = PAIRED ? 2 * is : is;
-  line_dft<kLanes>(
+  line_dft<kLanes, true>(
       f, buf, cl, lt, on, tw,
+      [&] {
+        fftcore::load_roots(tw, roots, f.L);
+        __syncthreads();
+      },
       [&](int r, int step, auto &a) {
         constexpr int R = sizeof(a) / sizeof(a[0]);
         r += in_add;
@@ -230,8 +255,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
   for (int c = c0; c < c1; ++c)
   {
     const float2 *sp = src + c * coil_stride + col;
-    line_dft<kLanes>(
-        f, buf, cl, lt, on, tw,
+    line_dft<kLanes, false>(
+        f, buf, cl, lt, on, tw, [] {},
         [&](int r, int step, auto &a) {
           constexpr int R = sizeof(a) / sizeof(a[0]);
 #pragma unroll
@@ -337,8 +362,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
   }
   __syncthreads();
   const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
-  line_dft<kRowPitch>(
-      f, buf, cl, lt, ln0 + cl < rows * C, tw,
+  line_dft<kRowPitch, false>(
+      f, buf, cl, lt, ln0 + cl < rows * C, tw, [] {},
       [&](int r, int step, auto &a) {
         constexpr int R = sizeof(a) / sizeof(a[0]);
         r += in_add;
@@ -422,8 +447,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks)
   const int cl = threadIdx.x % kLanes, lt = threadIdx.x / kLanes;
   const float2 *sp =
       grid + (size_t)c0 * g.grid_count + (size_t)row * f.L * pitch + cl;
-  line_dft<kRowPitch>(
-      f, buf, cl, lt, c0 + cl < C, tw,
+  line_dft<kRowPitch, false>(
+      f, buf, cl, lt, c0 + cl < C, tw, [] {},
       [&](int r, int step, auto &a) {
         constexpr int R = sizeof(a) / sizeof(a[0]);
         // FFT input n holds cell (n + floor(G / 2)) mod G
