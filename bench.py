@@ -437,34 +437,35 @@ def run_gpu_arm(args, rank, world, dist):
     G_cells = int(np.prod([v for v in g.grid_dims if v]))
     dim = len(dims)
     peak, src = peaks()
-    # algorithmic bytes per launch of the two gridding kernels.  General
-    # grids: k-space (8 B per sample per coil), coordinates (4 B per axis
-    # per sample) and the oversampled grid (8 B per cell per coil), read or
-    # written once.  Power-of-two grids (this workload) run
-    # k_forward_tma_groups (the same bytes) and k_adjoint_spmm_xfft, which
-    # reads the sorted k-space, the interpolation matrix (8 B per entry,
-    # kw^d entries per sample) and the row offsets (4 B per cell) and writes
-    # the x-transformed rows (8 B per coil per kept output, G / G_x * N_x
-    # per coil).
+    # algorithmic bytes of the two gridding stages: k-space (8 B per sample
+    # per coil), coordinates (4 B per axis per sample) and the oversampled
+    # grid (8 B per cell per coil), read or written once.  The column spread
+    # (k_tile_spread and the sums of its partial columns) writes the grid;
+    # small power-of-two adjoints run k_adjoint_spmm_xfft instead, which
+    # reads the interpolation matrix (8 B per entry, kw^d entries per sample)
+    # and the row offsets (4 B per cell) and writes the x-transformed rows
+    # (8 B per coil per kept output, G / G_x * N_x per coil).
     gbytes = 8 * M * C + 4 * dim * M + 8 * G_cells * C
     pow2 = all((v & (v - 1)) == 0 for v in g.grid_dims if v)
-    if pow2:
+    # launches of an adjoint without the column spread: gather, spread with
+    # the x transform and the other axes' passes (power-of-two grids), or
+    # gather, spread and the elementwise pass around cuFFT
+    columns = (stages["adj"][0]["launches"] > (dim + 1 if pow2 else 3))
+    fwd_kernel = ("k_forward_tma_groups" if dim == 3 else "k_forward_tma")
+    kernels = {fwd_kernel: ("forward interpolation",
+                            avg("fwd", "gridding_ms"), gbytes)}
+    if columns:
+        kernels["k_tile_spread"] = ("adjoint spread",
+                                    avg("adj", "gridding_ms"), gbytes)
+    elif pow2:
         nx_rows = G_cells // g.grid_dims[0] * dims[0]
-        abytes = (8 * M * C + 8 * M * inp["kw"] ** dim + 4 * G_cells +
-                  8 * C * nx_rows)
-        kernels = {
-            ("k_forward_tma_groups" if dim == 3 else "k_forward_tma"):
-                ("forward interpolation", avg("fwd", "gridding_ms"), gbytes),
-            "k_adjoint_spmm_xfft": ("adjoint spread + x transform",
-                                    avg("adj", "gridding_ms"), abytes),
-        }
+        kernels["k_adjoint_spmm_xfft"] = (
+            "adjoint spread + x transform", avg("adj", "gridding_ms"),
+            8 * M * C + 8 * M * inp["kw"] ** dim + 4 * G_cells +
+            8 * C * nx_rows)
     else:
-        kernels = {
-            "k_forward_interp": ("forward interpolation",
-                                 avg("fwd", "gridding_ms"), gbytes),
-            "k_adjoint_spmm": ("adjoint gridding", avg("adj", "gridding_ms"),
-                               gbytes),
-        }
+        kernels["k_adjoint_spmm"] = ("adjoint gridding",
+                                     avg("adj", "gridding_ms"), gbytes)
     rooflines = []
     for kname, (what, kms, nbytes) in kernels.items():
         ach = nbytes / (kms * 1e-3) / 1e9
